@@ -261,6 +261,8 @@ struct mo_ed_ctx {
     // square-lattice band of the DMFT self-consistency (mo_ed_set_band_structure)
     moed::DevBuf d_hk;
     int nq = 0;
+    moed::DevBuf d_hkw;        // its inequivalent k points, by weight (k_delta_new)
+    int hkw_end[4] = {0, 0, 0, 0};
 
     // scratch
     moed::DevBuf scratch_a, scratch_b, scratch_part;

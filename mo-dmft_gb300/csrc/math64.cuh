@@ -1,0 +1,36 @@
+// math64.cuh -- FP64 device arithmetic shared by the kernels.
+//
+// GB300 issues an FP64 warp instruction every 64 cycles per sub-partition, so
+// these helpers count FP64 instructions and use the integer and FP32 pipes
+// where that is exact.
+#pragma once
+
+#include <cuda_runtime.h>
+
+namespace moed {
+
+// 1/d for d > 0 from an FP32 seed y0 = rcp.approx(d) refined by one
+// third-order step of the Newton-Raphson family for the reciprocal,
+//   y1 = y0 + y0 (e + e^2),  e = 1 - d y0,
+// the truncated series y0 / (1 - e) = y0 (1 + e + e^2 + ...).  d is narrowed
+// to FP32 by truncating its significand (relative error < 2^-23) and the seed
+// widened back exactly, both with integer operations, so the FP64 pipe sees
+// only the three FMAs.  The seed's relative error |e| is below 2^-21, the
+// truncation error |e|^3 < 2^-63, and y1 is within one ulp of 1/d.  Outside
+// [2^-125, 2^126) (and for d <= 0, non-finite d) it is the IEEE division.
+__device__ __forceinline__ double rcp_pos(double d)
+{
+    const long long b = __double_as_longlong(d);
+    const int ex = (int)(b >> 52);                          // biased exponent (sign bit 0)
+    if ((unsigned)(ex - 898) > 250u) return 1.0 / d;        // FP32 exponent ex - 896 outside [2, 252]
+    const float df = __int_as_float(((ex - 896) << 23) | (int)((b >> 29) & 0x7fffff));
+    float yf;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(yf) : "f"(df));
+    const int fb = __float_as_int(yf);                      // a normal float: 1/df in (2^-126, 2^125]
+    const double y0 = __longlong_as_double(((long long)(((fb >> 23) & 0xff) + 896) << 52) |
+                                           ((long long)(fb & 0x7fffff) << 29));
+    const double e = fma(-d, y0, 1.0);
+    return fma(y0, fma(e, e, e), y0);
+}
+
+}  // namespace moed

@@ -9,7 +9,8 @@ namespace moed {
 
 void DevBuf::release()
 {
-    if (p) cudaFree(p);
+    if (slab) slab.reset();
+    else if (p) cudaFree(p);
     p = nullptr;
     bytes = 0;
 }
@@ -37,6 +38,34 @@ int dev_alloc(mo_ed_ctx *ctx, DevBuf &b, size_t bytes)
         return cuda_fail(ctx, e, "cudaMalloc");
     }
     b.bytes = bytes;
+    return MO_ED_OK;
+}
+
+int dev_alloc_slab(mo_ed_ctx *ctx, DevBuf *b, int n, size_t bytes)
+{
+    const size_t step = (bytes + 255) & ~(size_t)255;
+    DevBuf all;
+    if (int rc = dev_alloc(ctx, all, step * (size_t)n)) return rc;
+    std::shared_ptr<void> own(all.p, [](void *q) { cudaFree(q); });
+    char *base = (char *)all.p;
+    all.p = nullptr;
+    for (int i = 0; i < n; ++i) {
+        b[i].release();
+        b[i].p = base + step * (size_t)i;
+        b[i].bytes = bytes;
+        b[i].slab = own;
+    }
+    return MO_ED_OK;
+}
+
+int ensure_pinned(mo_ed_ctx *ctx, size_t bytes)
+{
+    if (ctx->pinned_bytes >= bytes) return MO_ED_OK;
+    if (ctx->pinned) cudaFreeHost(ctx->pinned);
+    ctx->pinned = nullptr;
+    ctx->pinned_bytes = 0;
+    MOED_CUDA(ctx, cudaMallocHost(&ctx->pinned, bytes));
+    ctx->pinned_bytes = bytes;
     return MO_ED_OK;
 }
 
@@ -136,6 +165,7 @@ int mo_ed_destroy(mo_ed_ctx *ctx)
     ctx->species.clear();
     ctx->states.clear();
     if (ctx->d_mdl) cudaFree(ctx->d_mdl);
+    if (ctx->pinned) cudaFreeHost(ctx->pinned);
     if (ctx->own_stream) cudaStreamDestroy(ctx->stream);
     delete ctx;
     return MO_ED_OK;

@@ -1221,6 +1221,108 @@ k_hv_down_rows(const __grid_constant__ HvBatch<TA> batch, int total)
     }
 }
 
+// ---------------------------------------------------------------------------
+// k_hv_row: one thread per element, one CTA per row (items of R = 1).
+// For small sectors the kernels above are bound by their set-up (barriers,
+// staging, tables of the item) and leave most threads without a column: a
+// sector of 4,900 elements took 10 us in FP32 and 12 us in FP64 on 18 of 256
+// or 512 threads per CTA.  Here the only barriers load the row's interspecies
+// diagonal; every term reads its operands directly (L1 / L2), the row's
+// down-spin moves as uniform loads, so a launch costs a few dependent loads.
+// ---------------------------------------------------------------------------
+template <typename TX, typename TA, typename TY, int NT>
+__global__ void __launch_bounds__(NT)
+k_hv_row(const __grid_constant__ HvBatch<TA> batch, const ModelDev *__restrict__ mdl)
+{
+    __shared__ TA s_cross[kMaxImp];
+    __shared__ unsigned s_pmask[kMaxImp];
+    __shared__ int s_t4[kMaxPair * kMaxImp];
+    __shared__ double s_red[NT / 32];
+    const int tid = threadIdx.x, nimp = mdl->nimp, npair = mdl->npair;
+    for (int i = tid; i < npair * nimp; i += NT) s_t4[i] = mdl->t4[i];
+    for (int i = tid; i < nimp; i += NT) s_pmask[i] = mdl->pairmask[i];
+    const TA Jc = (TA)mdl->J;
+    for (int item = blockIdx.x; item < batch.total_items; item += gridDim.x) {
+        int j = 0;
+        while (j + 1 < batch.njobs && item >= batch.job[j + 1].item0) ++j;
+        const HvJobT<TA> &jb = batch.job[j];
+        if (jb.active && *jb.active == 0) continue;
+        const int it = item - jb.item0, d = jb.items[it], ld = jb.ld;
+        const TX *__restrict__ x = (const TX *)jb.x;
+        const TX *__restrict__ xd = x + (size_t)d * ld;
+        TY *__restrict__ y = (TY *)jb.y + (size_t)d * ld;
+        const int dinf = __ldg(jb.dn_info + d), id = (dinf >> 8) & 0xff, dcnt = dinf & 0xff;
+        const TA ddiag = __ldg(jb.dn_diag + d);
+        __syncthreads();   // the previous row is done with s_cross and s_red
+        for (int i = tid; i < nimp; i += NT) s_cross[i] = (TA)mdl->cross[i * nimp + id];
+        __syncthreads();
+        double dacc = 0.0;
+        for (int u = tid; u < ld; u += NT) {
+            const int inf = __ldg(jb.up_info + u), iu = (inf >> 8) & 0xff, cnt = inf & 0xff;
+            const TX xv = __ldg(xd + u);
+            TA acc = (__ldg(jb.up_diag + u) + ddiag + s_cross[iu]) * (TA)xv;
+            // up-spin moves of the column, 4 at a time
+            const HopEnt<TA> *tab = jb.up_tab + (size_t)(u >> 2) * jb.up_hw * 4 + (u & 3);
+            for (int s0 = 0; s0 < cnt; s0 += 4) {
+                HopEnt<TA> e[4];
+                TX g[4];
+#pragma unroll
+                for (int t = 0; t < 4; ++t) e[t] = tab[4 * min(s0 + t, cnt - 1)];
+#pragma unroll
+                for (int t = 0; t < 4; ++t) g[t] = __ldg(xd + e[t].t);
+#pragma unroll
+                for (int t = 0; t < 4; ++t)
+                    if (s0 + t < cnt) acc += e[t].v * (TA)g[t];
+            }
+            // down-spin moves of the row
+            for (int s0 = 0; s0 < dcnt; s0 += 4) {
+                TA v[4];
+                TX g[4];
+#pragma unroll
+                for (int t = 0; t < 4; ++t) {
+                    const int s = min(s0 + t, dcnt - 1);
+                    v[t] = __ldg(jb.dn_val + (size_t)s * jb.nd + d);
+                    g[t] = __ldg(x + (size_t)__ldg(jb.dn_tgt + (size_t)s * jb.nd + d) * ld + u);
+                }
+#pragma unroll
+                for (int t = 0; t < 4; ++t)
+                    if (s0 + t < dcnt) acc += v[t] * (TA)g[t];
+            }
+            // spin-flip and pair hopping
+            unsigned pm = s_pmask[iu];
+            while (pm) {
+                const int p = __ffs(pm) - 1;
+                pm &= pm - 1;
+                const int e = s_t4[p * nimp + iu];
+                const TX *xu = x + u + (int)(short)(e & 0xffff);
+                const TA c = (e & 0x40000000) ? -Jc : Jc;
+                const int esf = s_t4[mdl->pair_rev[p] * nimp + id];   // spin-flip: T_{j<-i}(d)
+                const int eph = s_t4[p * nimp + id];                  // pair hop:  T_{i<-j}(d)
+                if (esf < 0) {
+                    const TX g = __ldg(xu + (size_t)(d + (int)(short)(esf & 0xffff)) * ld);
+                    acc += ((esf & 0x40000000) ? -c : c) * (TA)g;
+                }
+                if (eph < 0) {
+                    const TX g = __ldg(xu + (size_t)(d + (int)(short)(eph & 0xffff)) * ld);
+                    acc += ((eph & 0x40000000) ? -c : c) * (TA)g;
+                }
+            }
+            y[u] = (TY)acc;
+            if (jb.dot_partial) dacc += (double)((TA)xv * (TA)(TY)acc);
+        }
+        if (jb.dot_partial) {
+            for (int off = 16; off > 0; off >>= 1) dacc += __shfl_down_sync(0xffffffffu, dacc, off);
+            if ((tid & 31) == 0) s_red[tid >> 5] = dacc;
+            __syncthreads();
+            if (tid == 0) {
+                double t = 0.0;
+                for (int w = 0; w < NT / 32; ++w) t += s_red[w];
+                jb.dot_partial[it] = t;
+            }
+        }
+    }
+}
+
 template <typename TX, typename TA, int R>
 static size_t dyn_smem_bytes_async(int ld, const ModelDev &m, const DescGeom &g)
 {
@@ -1240,7 +1342,7 @@ static size_t dyn_smem_bytes_async(int ld, const ModelDev &m, const DescGeom &g)
 // (scratch vectors, CUDA events on the context stream) and keeps the fastest.
 struct HvVariant {
     int R, NT, MINB;
-    // 0: k_hv; 1: k_hv_async (double-buffered asynchronous stage);
+    // 0: k_hv, or k_hv_row when R = 1; 1: k_hv_async (double-buffered asynchronous stage);
     // 2 / 3: split, k_hv_down on 128- / 64-byte row slices + k_hv_async<SPLIT>;
     // 4: split, k_hv_down_rows (row AXPYs from L2) + k_hv_async<SPLIT>
     int staged;
@@ -1248,9 +1350,11 @@ struct HvVariant {
 static const HvVariant kVarF32[] = {{3, 512, 2, 0}, {4, 256, 2, 0}, {6, 512, 1, 0}, {3, 256, 3, 0},
                                     {8, 512, 1, 0}, {4, 512, 1, 1}, {3, 512, 1, 1}, {2, 512, 2, 1},
                                     {2, 256, 2, 1}, {3, 512, 1, 2}, {4, 512, 1, 2}, {3, 512, 1, 3},
-                                    {3, 512, 1, 4}, {4, 512, 1, 4}, {4, 512, 1, 4}};
+                                    {3, 512, 1, 4}, {4, 512, 1, 4}, {4, 512, 1, 4}, {1, 128, 8, 0}};
 static const HvVariant kVarF64[] = {{2, 256, 2, 0}, {3, 256, 1, 0}, {2, 512, 1, 0}, {2, 512, 1, 1},
-                                    {4, 512, 1, 1}, {2, 512, 1, 2}, {2, 512, 1, 3}, {2, 512, 1, 4}};
+                                    {4, 512, 1, 1}, {2, 512, 1, 2}, {2, 512, 1, 3}, {2, 512, 1, 4}, {1, 128, 8, 0}};
+static const int kRowVarF32 = 15, kRowVarF64 = 8;   // k_hv_row
+static const int kSmallVarF32 = 8;                   // k_hv_async<2, 256>: two CTAs per SM
 static const int kNVarF32 = sizeof(kVarF32) / sizeof(kVarF32[0]);
 static const int kNVarF64 = sizeof(kVarF64) / sizeof(kVarF64[0]);
 
@@ -1484,6 +1588,20 @@ static int launch_batch_rows(mo_ed_ctx *ctx, const HvBatch<TA> &b0)
     return launch_batch_async<TX, TA, TY, R, NT, MINB, true>(ctx, b);
 }
 
+// One element per thread (k_hv_row), one CTA per row.
+constexpr int kRowNT = 128;
+template <typename TX, typename TA, typename TY>
+static int launch_batch_row(mo_ed_ctx *ctx, const HvBatch<TA> &b)
+{
+    if (b.total_items <= 0) return MO_ED_OK;
+    for (int i = 0; i < b.njobs; ++i)
+        if (!b.job[i].items) return fail(ctx, MO_ED_ERR_STATE, "H*v item table missing");
+    const int grid = std::min(b.total_items, ctx->num_sms * 16);   // 16 CTAs of 128 threads fill an SM
+    k_hv_row<TX, TA, TY, kRowNT><<<grid, kRowNT, 0, ctx->stream>>>(b, ctx->d_mdl);
+    MOED_CHECK_LAUNCH(ctx);
+    return MO_ED_OK;
+}
+
 // Whether the split kernel fits every down-spin block of the model (any
 // electron count: at most dblk_bound rows and dblk_mv_bound moves).
 static bool split_fits(const mo_ed_ctx *ctx, size_t wb, size_t ent_bytes)
@@ -1546,7 +1664,8 @@ static int launch_variant(mo_ed_ctx *ctx, int kind, int v, const HvBatch<TA> &b)
         case 11: return launch_batch_split<float, float, float, 3, 512, 1, 64>(ctx, b);
         case 12: return launch_batch_rows<float, float, float, 3, 512, 1>(ctx, b);
         case 13: return launch_batch_rows<float, float, float, 4, 512, 1>(ctx, b);
-        default: return launch_batch_rows<float, float, float, 4, 512, 1, 4>(ctx, b);   // 2,048-column tiles
+        case 14: return launch_batch_rows<float, float, float, 4, 512, 1, 4>(ctx, b);   // 2,048-column tiles
+        default: return launch_batch_row<float, float, float>(ctx, b);
         }
     } else if (kind == HV_F64) {
         switch (v) {
@@ -1557,7 +1676,8 @@ static int launch_variant(mo_ed_ctx *ctx, int kind, int v, const HvBatch<TA> &b)
         case 4: return launch_batch_async<double, double, double, 4, 512>(ctx, b);
         case 5: return launch_batch_split<double, double, double, 2, 512, 1, 128>(ctx, b);
         case 6: return launch_batch_split<double, double, double, 2, 512, 1, 64>(ctx, b);
-        default: return launch_batch_rows<double, double, double, 2, 512, 1>(ctx, b);
+        case 7: return launch_batch_rows<double, double, double, 2, 512, 1>(ctx, b);
+        default: return launch_batch_row<double, double, double>(ctx, b);
         }
     } else {
         switch (v) {
@@ -1568,7 +1688,8 @@ static int launch_variant(mo_ed_ctx *ctx, int kind, int v, const HvBatch<TA> &b)
         case 4: return launch_batch_async<float, double, double, 4, 512>(ctx, b);
         case 5: return launch_batch_split<float, double, double, 2, 512, 1, 128>(ctx, b);
         case 6: return launch_batch_split<float, double, double, 2, 512, 1, 64>(ctx, b);
-        default: return launch_batch_rows<float, double, double, 2, 512, 1>(ctx, b);
+        case 7: return launch_batch_rows<float, double, double, 2, 512, 1>(ctx, b);
+        default: return launch_batch_row<float, double, double>(ctx, b);
         }
     }
 }
@@ -1693,7 +1814,11 @@ int hv_prepare(mo_ed_ctx *ctx, const Sector &s, int kind, int *v_out, int *R_out
     if (it != ctx->hv_choice.end()) {
         v = it->second;
     } else if (s.Dpad() < kTuneMinElems) {
-        v = 0;   // small sector: timing the variants would cost more than it saves
+        // small sector: timing the variants would cost more than it saves.
+        // k_hv_row against the best staged variant, us: FP32 8.3 : 8.3 at
+        // 15,876 elements, 10.3 : 8.3 at 63,504, 22.9 : 14.5 at 213,444; FP64
+        // 7.4 : 9.1 at 4,900, 12.4 : 12.4 at 63,504, 34.9 : 37.1 at 213,444.
+        v = kind != HV_F32 ? kRowVarF64 : s.D() < (1 << 15) ? kRowVarF32 : kSmallVarF32;
         ctx->hv_choice[key] = v;
         ctx->hv_times[key].assign(nvariants(kind), -1.0f);
     } else {
@@ -1762,6 +1887,45 @@ int hv_single(mo_ed_ctx *ctx, const Sector &s, int kind, const void *x, void *y)
     int v;
     if (int rc = hv_prepare(ctx, s, kind, &v, nullptr)) return rc;
     return launch_one(ctx, s, kind, v, x, y);
+}
+
+template <typename TA>
+static int multi_jobs(mo_ed_ctx *ctx, const Sector &s, int kind, int v, int n, const void *const *x, void *const *y)
+{
+    std::vector<HvJobT<TA>> jobs(n);
+    for (int i = 0; i < n; ++i) hv_fill_job<TA>(ctx, s, variant(kind, v).R, x[i], y[i], jobs[i]);
+    return hv_run_jobs<TA>(ctx, kind, v, jobs.data(), n);
+}
+
+int hv_multi(mo_ed_ctx *ctx, const Sector &s, int kind, int n, const void *const *x, void *const *y)
+{
+    int v;
+    if (int rc = hv_prepare(ctx, s, kind, &v, nullptr)) return rc;
+    return kind == HV_F32 ? multi_jobs<float>(ctx, s, kind, v, n, x, y) : multi_jobs<double>(ctx, s, kind, v, n, x, y);
+}
+
+int hv_dot_parts(mo_ed_ctx *ctx, const Sector &s, int kind, int *nparts)
+{
+    int v, R;
+    if (int rc = hv_prepare(ctx, s, kind, &v, &R)) return rc;
+    *nparts = s.dn->nitems.at(R);
+    return MO_ED_OK;
+}
+
+int hv_single_dot(mo_ed_ctx *ctx, const Sector &s, int kind, const void *x, void *y, double *dot)
+{
+    int v;
+    if (int rc = hv_prepare(ctx, s, kind, &v, nullptr)) return rc;
+    if (kind == HV_F32) {
+        HvJobT<float> j;
+        hv_fill_job<float>(ctx, s, variant(kind, v).R, x, y, j);
+        j.dot_partial = dot;
+        return hv_launch_f32(ctx, v, &j, 1);
+    }
+    HvJobT<double> j;
+    hv_fill_job<double>(ctx, s, variant(kind, v).R, x, y, j);
+    j.dot_partial = dot;
+    return hv_launch_f64(ctx, kind, v, &j, 1);
 }
 
 }  // namespace moed

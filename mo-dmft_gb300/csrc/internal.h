@@ -178,10 +178,11 @@ struct HvJobT {
 struct DevBuf {              // owning device allocation (move-only)
     void *p = nullptr;
     size_t bytes = 0;
+    std::shared_ptr<void> slab;   // set: p is a part of this allocation, shared with others
     DevBuf() = default;
     DevBuf(const DevBuf &) = delete;
     DevBuf &operator=(const DevBuf &) = delete;
-    DevBuf(DevBuf &&o) noexcept : p(o.p), bytes(o.bytes)
+    DevBuf(DevBuf &&o) noexcept : p(o.p), bytes(o.bytes), slab(std::move(o.slab))
     {
         o.p = nullptr;
         o.bytes = 0;
@@ -192,6 +193,7 @@ struct DevBuf {              // owning device allocation (move-only)
             release();
             p = o.p;
             bytes = o.bytes;
+            slab = std::move(o.slab);
             o.p = nullptr;
             o.bytes = 0;
         }
@@ -238,6 +240,8 @@ struct mo_ed_ctx {
     std::vector<int> cpl_orb, cpl_bath;  // nonzero couplings in reference loop order
     std::vector<double> cpl_val;
     std::vector<int> site_subsys;  // conserved subsystem (orbital + coupled bath levels) of each site
+    // the model can have exactly degenerate levels within a sector
+    bool degenerate = false;
     int dblk_bound = 0;            // largest down-spin block over every electron count
     int dblk_mv_bound = 0;         // most hybridisation moves in one such block
     std::map<int, std::unique_ptr<moed::Species>> species;  // by N
@@ -269,6 +273,12 @@ struct mo_ed_ctx {
     // eigensolver workspace reused across sectors (Krylov vectors of sectors
     // up to 64 MB per vector, and the projected-problem arrays)
     std::vector<moed::DevBuf> trl_pool, trl_small, rr_pool;
+    // eigs.cu: chunks of Krylov vectors kept between solves (at most
+    // kKryPoolBytes together), small arrays, and pinned host memory for the
+    // coefficients read while the next steps run
+    std::vector<moed::DevBuf> kry_pool, kry_small;
+    void *pinned = nullptr;
+    size_t pinned_bytes = 0;
     // autotuned H*v tile shape per (kind, Nup, Ndn), and the timings (ms) of
     // every shape measured when it was chosen (negative: did not fit)
     std::map<long long, int> hv_choice;
@@ -299,6 +309,9 @@ int cuda_fail(mo_ed_ctx *ctx, cudaError_t e, const char *what);
 
 int dev_alloc(mo_ed_ctx *ctx, DevBuf &b, size_t bytes);
 int ensure(mo_ed_ctx *ctx, DevBuf &b, size_t bytes);
+// n buffers of `bytes` each in one allocation, which goes with the last of them
+int dev_alloc_slab(mo_ed_ctx *ctx, DevBuf *b, int n, size_t bytes);
+int ensure_pinned(mo_ed_ctx *ctx, size_t bytes);
 // host vector in the reference layout (D contiguous) <-> device vector in the
 // padded layout (ndown rows of stride ld, zero pads); es = element size.
 int upload_padded(mo_ed_ctx *ctx, const Sector &s, const void *host, void *dev, size_t es);
@@ -350,6 +363,11 @@ int hv_lookup(mo_ed_ctx *ctx, const Sector &s, int kind, int *v, int *R);
 int hv_set_variant(mo_ed_ctx *ctx, const Sector &s, int kind, int v);
 // Convenience: one vector, jobs staged through scratch.
 int hv_single(mo_ed_ctx *ctx, const Sector &s, int kind, const void *x, void *y);
+// n vectors of one sector in as few launches as the batch allows.
+int hv_multi(mo_ed_ctx *ctx, const Sector &s, int kind, int n, const void *const *x, void *const *y);
+// y = H x with the partials of x . y in dot[0 .. hv_dot_parts); kind HV_F32 or HV_F64.
+int hv_dot_parts(mo_ed_ctx *ctx, const Sector &s, int kind, int *nparts);
+int hv_single_dot(mo_ed_ctx *ctx, const Sector &s, int kind, const void *x, void *y, double *dot);
 
 // ---- Krylov (krylov.cu) -----------------------------------------------------
 int lanczos_reference(mo_ed_ctx *ctx, const Sector &s, const double *h_vec, int nstep,

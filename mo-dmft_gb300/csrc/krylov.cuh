@@ -54,6 +54,21 @@ int lz_run(mo_ed_ctx *ctx, LzBatch &b, std::vector<std::vector<double>> &a,
 // FP64 sum of x*y over n elements (x, y of the given precisions), into *d_out.
 int dot_dev(mo_ed_ctx *ctx, int prec_x, const void *x, int prec_y, const void *y, long long n,
             double *d_out);
+// eigs.cu: the lowest eigenpairs by one long Lanczos run with periodic
+// reorthogonalisation.  *done = false (and MO_ED_OK) when the sector or the
+// options are not its case, or it gave up: the caller uses thick restarts.
+template <typename T>
+int plz_solve(mo_ed_ctx *ctx, const Sector &s, int nev, std::vector<double> &vals, std::vector<DevBuf> *vecs,
+              bool *done);
+template <typename T>
+struct VPtrs;
+// eigs.cu: Ritz vectors X_c = sum_l V_l Y[c * m + l] (c < nout, Y on the
+// device), then the FP64 Rayleigh-Ritz on their span: vals[0 .. nout), and the
+// vectors into *vecs if not null; entries nout .. nev of vals are DBL_MAX.
+template <typename T>
+int ritz_pairs(mo_ed_ctx *ctx, const Sector &s, const VPtrs<T> &V, int m, const double *d_Y, int nout, int nev,
+               long long matvecs, std::vector<double> &vals, std::vector<DevBuf> *vecs);
+
 int convert_f64_to_f32(mo_ed_ctx *ctx, const double *in, float *out, long long n);
 int convert_f32_to_f64(mo_ed_ctx *ctx, const float *in, double *out, long long n);
 

@@ -33,4 +33,15 @@ __device__ __forceinline__ double rcp_pos(double d)
     return fma(y0, fma(e, e, e), y0);
 }
 
+// (double)f by integer operations (a conversion instruction would take a slot
+// of the FP64 pipe); denormals, infinities and NaN take the conversion.
+__device__ __forceinline__ double widen(float f)
+{
+    const unsigned b = __float_as_uint(f);
+    if ((b << 1) == 0u) return __hiloint2double((int)b, 0);
+    if (((b & 0x7f800000u) - 0x00800000u) >= 0x7f000000u) return (double)f;
+    return __hiloint2double((int)((((b & 0x7fffffffu) >> 3) + 0x38000000u) | (b & 0x80000000u)), (int)(b << 29));
+}
+__device__ __forceinline__ double widen(double f) { return f; }
+
 }  // namespace moed

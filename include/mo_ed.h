@@ -153,9 +153,11 @@ int mo_ed_multiply_h_mixed_dev(mo_ed_ctx *ctx, int ne_up, int ne_down, const flo
  * reference has one CPU loop).  The first H*v of each (precision, Nup, Ndn)
  * times every variant on that sector and keeps the fastest; this call runs
  * the tuning if needed and reports *nvariant variants: shape[4*i..4*i+3] =
- * (rows per item, threads per CTA, CTAs per SM, kernel: 0 k_hv, 1 the
- * double-buffered staged k_hv_async, 2 / 3 split: k_hv_down over down-spin
- * blocks on 128- / 64-byte row slices, then k_hv_async for the other terms),
+ * (rows per item, threads per CTA, CTAs per SM, kernel: 0 k_hv, or k_hv_row
+ * with one row per item; 1 the staged kernels k_hv_async and k_hv_wide; 2 / 3
+ * split: k_hv_down over down-spin blocks on 128- / 64-byte row slices, then
+ * k_hv_async for the other terms; 4 split: k_hv_down_rows, then k_hv_async or
+ * k_hv_wide),
  * ms[i] (negative: does not fit this sector or model), and the *chosen
  * index.  Arrays hold capacity variants.  Pinning a split variant on a model
  * whose down-spin blocks do not fit one CTA fails with MO_ED_ERR_ARG. */

@@ -33,7 +33,8 @@
 // chunk-major table, one contiguous block per slot.
 //
 // k_hv_async (below): double-buffered asynchronous stage, conflict-free
-// scheduled up-spin gathers, precomputed item descriptors.
+// scheduled up-spin gathers, precomputed item descriptors.  k_hv_wide: the
+// FP32 successor of it for up to three orbitals.  k_hv_row: small sectors.
 //
 // Split (below): k_hv_down computes the down-spin hybridisation over
 // down-spin blocks x column slices from shared memory, or k_hv_down_rows as
@@ -1323,6 +1324,299 @@ k_hv_row(const __grid_constant__ HvBatch<TA> batch, const ModelDev *__restrict__
     }
 }
 
+// ---------------------------------------------------------------------------
+// k_hv_wide: FP32, up to three orbitals, R = 4 or 8 rows per item.
+// The same fused sum as k_hv_async, arranged so that one schedule entry and
+// one down-spin address serve more elements:
+//   * the staged rows lie in planes of 16 bytes per column (4 rows each): a
+//     move of a column reads 4 rows with one 16-byte load, where k_hv_async
+//     took one 4-byte load per row;
+//   * a lane owns two neighbouring columns: 8-byte loads of the down-spin
+//     rows and stores of y, one row address for both, one 16-byte load for the
+//     schedule entries of both;
+//   * the quarter warps' targets of a slot fall in 8 different bank groups
+//     (species_wide), so the 16-byte loads have no conflicts;
+//   * a bath group of 2 or 3 rows sits in rows 0-2 of a plane; T_{i<-j} of the
+//     up spin couples its rows pairwise (spin-flip one way, pair hopping the
+//     other, the same sign), so the 4-operator terms are, per transition of
+//     the column, one 16-byte load of the partner column and 6 FMAs with three
+//     coefficients from a table of the model, without branches.
+// Bound by shared-memory wavefronts and their latency (ncu, 15 million
+// elements: 55 % of the LSU pipe, DRAM at 19 %): a slot serves the lanes that
+// have a move in it, 58 % of them.  Ground sector of 3 orbitals x 4 levels, 41
+// million elements: R = 8 after k_hv_down_rows 320 us (of it k_hv_wide 216),
+// two CTAs of R = 4 fused 345 us, R = 4 split 335 us; k_hv_async<SPLIT, 4> 463.
+// Tried and not kept: more slots or moves in flight at fewer warps (350-550
+// us, registers), skipping the lanes without a move by predicate (the same).
+// ---------------------------------------------------------------------------
+struct WideLayout {        // dynamic shared memory, in bytes
+    int plane, cross, mv, jtab, dm;
+};
+
+__device__ __forceinline__ float4 wide_ld(const unsigned char *p) { return *reinterpret_cast<const float4 *>(p); }
+
+// SPLIT: k_hv_down_rows has written the down-spin hybridisation into y; this
+// kernel adds the other terms.  SB: schedule slots in flight; DB: down-spin
+// moves of 4 rows in flight.
+template <int R, int NT, int MINB, bool SPLIT, int SB, int DB>
+__global__ void __launch_bounds__(NT, MINB)
+k_hv_wide(const __grid_constant__ HvBatch<float> batch, const ModelDev *__restrict__ mdl, const WideLayout L)
+{
+    constexpr int NW = NT / 32, NP = R / 4;
+    extern __shared__ __align__(16) unsigned char smem_wide[];
+    float *const s_cross = reinterpret_cast<float *>(smem_wide + L.cross);   // [nimp][R]: interspecies + row diagonal
+    HopEnt<float> *const s_mv = reinterpret_cast<HopEnt<float> *>(smem_wide + L.mv);   // [R][dm]: {row offset, coupling}
+    const float4 *const s_j = reinterpret_cast<const float4 *>(smem_wide + L.jtab);    // [2][nimp][2]
+    __shared__ int s_d[R], s_cnt[R], s_type[NP], s_most[NP];   // s_most: largest count of a plane's rows
+    __shared__ double s_red[NW];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int nimp = mdl->nimp, npair = mdl->npair, norb = mdl->norb;
+
+    // 4-operator table: for a group with ty + 1 impurity electrons and column
+    // pattern iu, transition t: coefficients of the row pairs (0,1), (0,2),
+    // (1,2) and the byte offset of the partner column
+    if (tid < 2 * nimp) {
+        const int ty = tid / nimp, iu = tid - ty * nimp;
+        int nt = 0;
+        float4 e[2] = {make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f)};
+        for (int p = 0; p < npair && nt < 2; ++p) {
+            const int tu = mdl->t4[p * nimp + iu];   // T_{i<-j} of the up spin
+            if (tu >= 0) continue;
+            float c[3] = {0.f, 0.f, 0.f};
+            if (ty + 1 < norb) {
+                int idx = 0;
+                for (int a = 0; a < nimp; ++a) {     // patterns of the group, in rank order
+                    if (__popc(a) != ty + 1) continue;
+                    const int td = mdl->t4[p * nimp + a];   // T_{i<-j} of the down spin on pattern a
+                    if (td < 0) {
+                        const int b = idx + (int)(short)(td & 0xffff);
+                        const float v = (float)mdl->J * ((((tu ^ td) & 0x40000000) != 0) ? -1.f : 1.f);
+                        c[min(idx, b) + max(idx, b) - 1] = v;   // (0,1) 0, (0,2) 1, (1,2) 2
+                    }
+                    ++idx;
+                }
+            }
+            e[nt] = make_float4(c[0], c[1], c[2], __int_as_float((int)(short)(tu & 0xffff) * 16));
+            ++nt;
+        }
+        float4 *o = const_cast<float4 *>(s_j) + 2 * tid;
+        o[0] = e[0];
+        o[1] = e[1];
+    }
+
+    int cur = hv_next_item(batch, (int)blockIdx.x);
+    while (cur >= 0) {
+        const HvJobT<float> &jb = batch.job[hv_find_job(batch, cur)];
+        const int it = cur - jb.item0, ld = jb.ld, nd = jb.nd;
+        const float *__restrict__ x = (const float *)jb.x;
+        float *__restrict__ y = (float *)jb.y;
+        const int *const rows = jb.items + (size_t)it * R;
+        __syncthreads();   // the previous item is done with shared memory
+        if (tid < R) {
+            const int d = __ldg(rows + tid);
+            const int inf = d >= 0 ? __ldg(jb.dn_info + d) : 0;
+            s_d[tid] = d;
+            s_cnt[tid] = inf & 0xff;
+            if ((tid & 3) == 0) {
+                const int pc = __popc((inf >> 8) & 0xff);
+                s_type[tid >> 2] = (d >= 0 && pc > 0 && pc < norb) ? pc : 0;
+            }
+            int most = inf & 0xff;
+            most = max(most, __shfl_xor_sync((1u << R) - 1u, most, 1));
+            most = max(most, __shfl_xor_sync((1u << R) - 1u, most, 2));
+            if ((tid & 3) == 0) s_most[tid >> 2] = most;
+        }
+        for (int i = tid; i < nimp * R; i += NT) {
+            const int iu = i / R, d = __ldg(rows + (i - iu * R));
+            const int id = d >= 0 ? (__ldg(jb.dn_info + d) >> 8) & 0xff : 0;
+            s_cross[i] = d >= 0 ? (float)mdl->cross[iu * nimp + id] + __ldg(jb.dn_diag + d) : 0.f;
+        }
+        if (!SPLIT)
+            for (int i = tid; i < R * jb.dn_maxcnt; i += NT) {
+                const int s = i / R, r = i - s * R, d = __ldg(rows + r);
+                if (d >= 0 && s < (__ldg(jb.dn_info + d) & 0xff)) {
+                    HopEnt<float> e;
+                    e.t = __ldg(jb.dn_tgt + (size_t)s * nd + d) * ld;
+                    e.v = __ldg(jb.dn_val + (size_t)s * nd + d);
+                    s_mv[r * L.dm + s] = e;
+                }
+            }
+        {   // stage: two neighbouring columns of R rows per thread
+            int dr[R];
+#pragma unroll
+            for (int r = 0; r < R; ++r) dr[r] = __ldg(rows + r);
+            for (int u = 2 * tid; u < ld; u += 2 * NT) {
+                float2 v[R];
+#pragma unroll
+                for (int r = 0; r < R; ++r)
+                    v[r] = dr[r] >= 0 ? __ldg(reinterpret_cast<const float2 *>(x + (size_t)dr[r] * ld + u))
+                                      : make_float2(0.f, 0.f);
+#pragma unroll
+                for (int p = 0; p < NP; ++p) {
+                    unsigned char *o = smem_wide + p * L.plane + 16 * u;
+                    *reinterpret_cast<float4 *>(o) = make_float4(v[4 * p].x, v[4 * p + 1].x, v[4 * p + 2].x, v[4 * p + 3].x);
+                    *reinterpret_cast<float4 *>(o + 16) = make_float4(v[4 * p].y, v[4 * p + 1].y, v[4 * p + 2].y, v[4 * p + 3].y);
+                }
+            }
+        }
+        const int nxt = hv_next_item(batch, cur + (int)gridDim.x);
+        if (nxt >= 0) {   // the next item's rows into L2, one 128-byte line per thread and turn
+            const HvJobT<float> &jn = batch.job[hv_find_job(batch, nxt)];
+            const int *const rn = jn.items + (size_t)(nxt - jn.item0) * R;
+            const int lines = jn.ld >> 5;
+            for (int i = tid; i < R * lines; i += NT) {
+                const int r = i / lines, d = __ldg(rn + r);
+                if (d >= 0)
+                    asm volatile("prefetch.global.L2 [%0];" ::"l"((const float *)jn.x + (size_t)d * jn.ld +
+                                                                  32 * (i - r * lines)));
+            }
+        }
+        __syncthreads();
+        const bool want_dot = jb.dot_partial != nullptr;
+        float part = 0.f;
+        const int nunit = (ld + 63) >> 6;
+        for (int c = warp; c < nunit; c += NW) {
+            const int u = 64 * c + 2 * lane;
+            const bool has = u < ld;             // ld is a multiple of 32: both columns or none
+            const int uc = has ? u : 0;
+            const int2 h = __ldg(jb.up_sched_hdr + c);
+            const float4 *ent = reinterpret_cast<const float4 *>(jb.up_sched + h.x) + lane;   // two entries per lane
+            float4 e[SB];
+#pragma unroll
+            for (int t = 0; t < SB; ++t) e[t] = t < h.y ? __ldg(ent + 32 * t) : make_float4(0.f, 0.f, 0.f, 0.f);
+            const int2 inf = __ldg(reinterpret_cast<const int2 *>(jb.up_info + uc));
+            const float2 ud = __ldg(reinterpret_cast<const float2 *>(jb.up_diag + uc));
+            const float *xu = x + uc;
+            float acc[2][R];
+            // down-spin rows, DB moves of 4 rows at a time; the first batch is in
+            // flight during the diagonal
+            float2 g[4][DB];
+            auto load_moves = [&](int r0, int s0) {
+#pragma unroll
+                for (int q = 0; q < 4; ++q)
+#pragma unroll
+                    for (int t = 0; t < DB; ++t) {
+                        g[q][t] = make_float2(0.f, 0.f);
+                        if (s0 + t < s_cnt[r0 + q])
+                            g[q][t] = __ldg(reinterpret_cast<const float2 *>(xu + (unsigned)s_mv[(r0 + q) * L.dm + s0 + t].t));
+                    }
+            };
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                float2 yp = make_float2(0.f, 0.f);
+                if constexpr (SPLIT) {
+                    const int d = s_d[r];
+                    if (has && d >= 0) yp = *reinterpret_cast<const float2 *>(y + (size_t)d * ld + u);
+                }
+                acc[0][r] = yp.x;
+                acc[1][r] = yp.y;
+            }
+            if constexpr (!SPLIT) load_moves(0, 0);
+            // diagonal and 4-operator terms
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                const int iu = ((k ? inf.y : inf.x) >> 8) & 0xff;
+                const float udk = k ? ud.y : ud.x;
+#pragma unroll
+                for (int p = 0; p < NP; ++p) {
+                    const unsigned char *S = smem_wide + p * L.plane + 16 * (uc + k);
+                    float *a = acc[k] + 4 * p;
+                    const float4 xa = wide_ld(S);
+                    const float4 ca = *reinterpret_cast<const float4 *>(s_cross + iu * R + 4 * p);
+                    a[0] += (udk + ca.x) * xa.x;
+                    a[1] += (udk + ca.y) * xa.y;
+                    a[2] += (udk + ca.z) * xa.z;
+                    a[3] += (udk + ca.w) * xa.w;
+                    const int ty = s_type[p];
+                    if (ty) {
+#pragma unroll
+                        for (int t = 0; t < 2; ++t) {
+                            const float4 j = s_j[((ty - 1) * nimp + iu) * 2 + t];
+                            const float4 v = wide_ld(S + __float_as_int(j.w));
+                            a[0] += j.x * v.y + j.y * v.z;
+                            a[1] += j.x * v.x + j.z * v.z;
+                            a[2] += j.y * v.x + j.z * v.y;
+                        }
+                    }
+                }
+            }
+            if constexpr (!SPLIT) {
+#pragma unroll
+                for (int p = 0; p < NP; ++p) {
+                    const int n = s_most[p];
+                    for (int s0 = 0; s0 < n; s0 += DB) {
+                        if (p > 0 || s0 > 0) load_moves(4 * p, s0);
+#pragma unroll
+                        for (int q = 0; q < 4; ++q)
+#pragma unroll
+                            for (int t = 0; t < DB; ++t)
+                                if (s0 + t < s_cnt[4 * p + q]) {
+                                    const float v = s_mv[(4 * p + q) * L.dm + s0 + t].v;
+                                    acc[0][4 * p + q] += v * g[q][t].x;
+                                    acc[1][4 * p + q] += v * g[q][t].y;
+                                }
+                    }
+                }
+            }
+            // up-spin moves: SB slots ahead
+            for (int s0 = 0; s0 < h.y; s0 += SB) {
+                float4 f[SB];
+#pragma unroll
+                for (int t = 0; t < SB; ++t)
+                    f[t] = s0 + SB + t < h.y ? __ldg(ent + 32 * (s0 + SB + t)) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+                for (int t = 0; t < SB; ++t) {
+#pragma unroll
+                    for (int k = 0; k < 2; ++k) {
+                        const unsigned char *S = smem_wide + __float_as_int(k ? e[t].z : e[t].x);
+                        const float v = k ? e[t].w : e[t].y;
+#pragma unroll
+                        for (int p = 0; p < NP; ++p) {
+                            const float4 ga = wide_ld(S + p * L.plane);
+                            float *a = acc[k] + 4 * p;
+                            a[0] += v * ga.x;
+                            a[1] += v * ga.y;
+                            a[2] += v * ga.z;
+                            a[3] += v * ga.w;
+                        }
+                    }
+                }
+#pragma unroll
+                for (int t = 0; t < SB; ++t) e[t] = f[t];
+            }
+            if (has) {
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    const int d = s_d[r];
+                    if (d >= 0) *reinterpret_cast<float2 *>(y + (size_t)d * ld + u) = make_float2(acc[0][r], acc[1][r]);
+                }
+                if (want_dot) {   // rows that are not there are staged as zeros
+#pragma unroll
+                    for (int k = 0; k < 2; ++k)
+#pragma unroll
+                        for (int p = 0; p < NP; ++p) {
+                            const float4 xa = wide_ld(smem_wide + p * L.plane + 16 * (u + k));
+                            const float *a = acc[k] + 4 * p;
+                            part += (xa.x * a[0] + xa.y * a[1]) + (xa.z * a[2] + xa.w * a[3]);
+                        }
+                }
+            }
+        }
+        if (want_dot) {
+            double dacc = (double)part;
+            for (int off = 16; off > 0; off >>= 1) dacc += __shfl_down_sync(0xffffffffu, dacc, off);
+            if (lane == 0) s_red[warp] = dacc;
+            __syncthreads();
+            if (tid == 0) {
+                double t = 0.0;
+                for (int w = 0; w < NW; ++w) t += s_red[w];
+                jb.dot_partial[it] = t;
+            }
+        }
+        cur = nxt;
+    }
+}
+
 template <typename TX, typename TA, int R>
 static size_t dyn_smem_bytes_async(int ld, const ModelDev &m, const DescGeom &g)
 {
@@ -1346,9 +1640,11 @@ struct HvVariant {
     // 2 / 3: split, k_hv_down on 128- / 64-byte row slices + k_hv_async<SPLIT>;
     // 4: split, k_hv_down_rows (row AXPYs from L2) + k_hv_async<SPLIT>
     int staged;
+    bool wide = false;   // k_hv_wide in the place of k_hv_async
+    int key() const { return wide ? kWideKey + R : R; }   // of the item table
 };
-static const HvVariant kVarF32[] = {{3, 512, 2, 0}, {4, 256, 2, 0}, {6, 512, 1, 0}, {3, 256, 3, 0},
-                                    {8, 512, 1, 0}, {4, 512, 1, 1}, {3, 512, 1, 1}, {2, 512, 2, 1},
+static const HvVariant kVarF32[] = {{4, 512, 2, 1, true}, {4, 256, 2, 0}, {6, 512, 1, 0}, {3, 256, 3, 0},
+                                    {8, 832, 1, 4, true}, {4, 512, 1, 1}, {3, 512, 1, 1}, {4, 512, 2, 4, true},
                                     {2, 256, 2, 1}, {3, 512, 1, 2}, {4, 512, 1, 2}, {3, 512, 1, 3},
                                     {3, 512, 1, 4}, {4, 512, 1, 4}, {4, 512, 1, 4}, {1, 128, 8, 0}};
 static const HvVariant kVarF64[] = {{2, 256, 2, 0}, {3, 256, 1, 0}, {2, 512, 1, 0}, {2, 512, 1, 1},
@@ -1411,7 +1707,10 @@ void hv_fill_job(const mo_ed_ctx *ctx, const Sector &s, int R, const void *x, vo
     j.dblk_max = s.dn->dblk_max;
     j.dblk_mvmax = s.dn->dblk_mvmax;
     j.tile0 = 0;
-    if (f32) {
+    if (f32 && R >= kWideKey) {
+        j.up_sched_hdr = s.up->wide_hdr;
+        j.up_sched = (const HopEnt<TA> *)s.up->wide_ent;
+    } else if (f32) {
         auto sf = s.up->sched_rf.find(R);
         j.up_sched = sf != s.up->sched_rf.end() ? (const HopEnt<TA> *)sf->second : nullptr;
     } else {
@@ -1561,11 +1860,9 @@ static int launch_batch_split(mo_ed_ctx *ctx, const HvBatch<TA> &b0)
 // Split H*v with the row-AXPY down pass: k_hv_down_rows writes the
 // down-spin hybridisation into y, then k_hv_async<SPLIT> adds the rest.
 constexpr int kRowsNT = 128;   // 512 CPT columns per tile
-template <typename TX, typename TA, typename TY, int R, int NT, int MINB, int CPT = 2>
-static int launch_batch_rows(mo_ed_ctx *ctx, const HvBatch<TA> &b0)
+template <typename TX, typename TA, typename TY, int CPT>
+static int launch_rows_pass(mo_ed_ctx *ctx, HvBatch<TA> &b)
 {
-    if (b0.total_items <= 0) return MO_ED_OK;
-    HvBatch<TA> b = b0;
     long long tiles = 0;
     for (int i = 0; i < b.njobs; ++i) {
         HvJobT<TA> &j = b.job[i];
@@ -1585,6 +1882,15 @@ static int launch_batch_rows(mo_ed_ctx *ctx, const HvBatch<TA> &b0)
         kd<<<grid, kRowsNT, 0, ctx->stream>>>(b, (int)tiles);
         MOED_CHECK_LAUNCH(ctx);
     }
+    return MO_ED_OK;
+}
+
+template <typename TX, typename TA, typename TY, int R, int NT, int MINB, int CPT = 2>
+static int launch_batch_rows(mo_ed_ctx *ctx, const HvBatch<TA> &b0)
+{
+    if (b0.total_items <= 0) return MO_ED_OK;
+    HvBatch<TA> b = b0;
+    if (int rc = launch_rows_pass<TX, TA, TY, CPT>(ctx, b)) return rc;
     return launch_batch_async<TX, TA, TY, R, NT, MINB, true>(ctx, b);
 }
 
@@ -1598,6 +1904,45 @@ static int launch_batch_row(mo_ed_ctx *ctx, const HvBatch<TA> &b)
         if (!b.job[i].items) return fail(ctx, MO_ED_ERR_STATE, "H*v item table missing");
     const int grid = std::min(b.total_items, ctx->num_sms * 16);   // 16 CTAs of 128 threads fill an SM
     k_hv_row<TX, TA, TY, kRowNT><<<grid, kRowNT, 0, ctx->stream>>>(b, ctx->d_mdl);
+    MOED_CHECK_LAUNCH(ctx);
+    return MO_ED_OK;
+}
+
+// shared memory of k_hv_wide for rows of up to ldmax columns
+static WideLayout wide_layout(int ldmax, int rows, const ModelDev &m, size_t *total)
+{
+    WideLayout L;
+    L.plane = 16 * ldmax;
+    L.dm = std::max(m.ncpl, 1);
+    L.cross = rows / 4 * L.plane;
+    L.mv = L.cross + (int)sizeof(float) * m.nimp * rows;
+    L.jtab = (int)align16((size_t)L.mv + sizeof(HopEnt<float>) * rows * (size_t)L.dm);
+    *total = (size_t)L.jtab + sizeof(float4) * 4 * (size_t)m.nimp;
+    return L;
+}
+
+template <int R, int NT, int MINB, bool SPLIT, int SB, int DB>
+static int launch_batch_wide(mo_ed_ctx *ctx, const HvBatch<float> &b0)
+{
+    if (b0.total_items <= 0) return MO_ED_OK;
+    if (ctx->mdl.norb > 3) return fail(ctx, MO_ED_ERR_ARG, "more orbitals than this H*v tile shape takes");
+    HvBatch<float> b = b0;
+    int ldmax = 0;
+    for (int i = 0; i < b.njobs; ++i) {
+        ldmax = std::max(ldmax, b.job[i].ld);
+        if (!b.job[i].items || !b.job[i].up_sched_hdr || !b.job[i].up_sched)
+            return fail(ctx, MO_ED_ERR_STATE, "H*v tables missing");
+    }
+    size_t smem = 0;
+    const WideLayout L = wide_layout(ldmax, R, ctx->mdl, &smem);
+    auto kern = k_hv_wide<R, NT, MINB, SPLIT, SB, DB>;
+    int per_sm = 0;
+    if (int rc = kernel_fit(ctx, kern, NT, smem, &per_sm)) return rc;
+    if (per_sm < 1) return fail(ctx, MO_ED_ERR_ARG, "sector rows too long for the shared-memory stage");
+    if (SPLIT)
+        if (int rc = launch_rows_pass<float, float, float, 2>(ctx, b)) return rc;
+    const int grid = std::min(b.total_items, ctx->num_sms * per_sm);
+    kern<<<grid, NT, smem, ctx->stream>>>(b, ctx->d_mdl, L);
     MOED_CHECK_LAUNCH(ctx);
     return MO_ED_OK;
 }
@@ -1650,14 +1995,14 @@ static int launch_variant(mo_ed_ctx *ctx, int kind, int v, const HvBatch<TA> &b)
     if constexpr (sizeof(TA) == 4) {
         (void)kind;
         switch (v) {
-        case 0: return launch_batch<float, float, float, 3, 512, 2>(ctx, b);
+        case 0: return launch_batch_wide<4, 512, 2, false, 2, 2>(ctx, b);
         case 1: return launch_batch<float, float, float, 4, 256, 2>(ctx, b);
         case 2: return launch_batch<float, float, float, 6, 512, 1>(ctx, b);
         case 3: return launch_batch<float, float, float, 3, 256, 3>(ctx, b);
-        case 4: return launch_batch<float, float, float, 8, 512, 1>(ctx, b);
+        case 4: return launch_batch_wide<8, 832, 1, true, 2, 1>(ctx, b);
         case 5: return launch_batch_async<float, float, float, 4, 512>(ctx, b);
         case 6: return launch_batch_async<float, float, float, 3, 512>(ctx, b);
-        case 7: return launch_batch_async<float, float, float, 2, 512, 2>(ctx, b);
+        case 7: return launch_batch_wide<4, 512, 2, true, 2, 1>(ctx, b);
         case 8: return launch_batch_async<float, float, float, 2, 256, 2>(ctx, b);
         case 9: return launch_batch_split<float, float, float, 3, 512, 1, 128>(ctx, b);
         case 10: return launch_batch_split<float, float, float, 4, 512, 1, 128>(ctx, b);
@@ -1726,7 +2071,7 @@ int hv_launch_f64(mo_ed_ctx *ctx, int kind, int v, const HvJobT<double> *jobs, i
 
 static int launch_one(mo_ed_ctx *ctx, const Sector &s, int kind, int v, const void *x, void *y)
 {
-    const int R = variant(kind, v).R;
+    const int R = variant(kind, v).key();
     if (kind == HV_F32) {
         HvJobT<float> j;
         hv_fill_job<float>(ctx, s, R, x, y, j);
@@ -1744,8 +2089,9 @@ static int prepare_variant(mo_ed_ctx *ctx, const Sector &s, int kind, int v)
     const HvVariant &h = variant(kind, v);
     const int *items;
     int n;
-    if (int rc = species_items(ctx, s.dn, h.R, &items, &n)) return rc;
+    if (int rc = species_items(ctx, s.dn, h.key(), &items, &n)) return rc;
     if (!h.staged) return MO_ED_OK;
+    if (h.wide) return species_wide(ctx, s.up);
     if (h.staged == 2 || h.staged == 3) {
         // the split kernel stages whole down-spin blocks: the largest block of
         // the model (any electron count) must fit one CTA's shared memory
@@ -1827,7 +2173,7 @@ int hv_prepare(mo_ed_ctx *ctx, const Sector &s, int kind, int *v_out, int *R_out
     }
     if (int rc = prepare_variant(ctx, s, kind, v)) return rc;
     if (v_out) *v_out = v;
-    if (R_out) *R_out = variant(kind, v).R;
+    if (R_out) *R_out = variant(kind, v).key();
     return MO_ED_OK;
 }
 
@@ -1862,9 +2208,11 @@ int hv_lookup(mo_ed_ctx *ctx, const Sector &s, int kind, int *v_out, int *R_out)
     if (it == ctx->hv_choice.end())
         return fail(ctx, MO_ED_ERR_STATE, "H*v tile shape of this sector not chosen yet");
     const HvVariant &h = variant(kind, it->second);
-    const int R = h.R;
+    const int R = h.key();
     bool ready = s.dn->items.count(R) != 0;
-    if (h.staged)
+    if (h.wide)
+        ready = ready && s.up->wide_ent != nullptr;
+    else if (h.staged)
         ready = ready && s.up->sched_rf.count(R) && s.dn->desc.count(R * 2 + (kind == HV_F32 ? 0 : 1));
     if (h.staged == 2 || h.staged == 3)
         ready = ready && s.dn->dblk_ptr != nullptr && s.dn->dblk_chunks.count(s.ld());
@@ -1893,7 +2241,7 @@ template <typename TA>
 static int multi_jobs(mo_ed_ctx *ctx, const Sector &s, int kind, int v, int n, const void *const *x, void *const *y)
 {
     std::vector<HvJobT<TA>> jobs(n);
-    for (int i = 0; i < n; ++i) hv_fill_job<TA>(ctx, s, variant(kind, v).R, x[i], y[i], jobs[i]);
+    for (int i = 0; i < n; ++i) hv_fill_job<TA>(ctx, s, variant(kind, v).key(), x[i], y[i], jobs[i]);
     return hv_run_jobs<TA>(ctx, kind, v, jobs.data(), n);
 }
 
@@ -1918,12 +2266,12 @@ int hv_single_dot(mo_ed_ctx *ctx, const Sector &s, int kind, const void *x, void
     if (int rc = hv_prepare(ctx, s, kind, &v, nullptr)) return rc;
     if (kind == HV_F32) {
         HvJobT<float> j;
-        hv_fill_job<float>(ctx, s, variant(kind, v).R, x, y, j);
+        hv_fill_job<float>(ctx, s, variant(kind, v).key(), x, y, j);
         j.dot_partial = dot;
         return hv_launch_f32(ctx, v, &j, 1);
     }
     HvJobT<double> j;
-    hv_fill_job<double>(ctx, s, variant(kind, v).R, x, y, j);
+    hv_fill_job<double>(ctx, s, variant(kind, v).key(), x, y, j);
     j.dot_partial = dot;
     return hv_launch_f64(ctx, kind, v, &j, 1);
 }

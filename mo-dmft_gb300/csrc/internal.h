@@ -105,6 +105,13 @@ struct Species {
     // no other lane of the slot uses, with coupling 0
     std::map<int, HopEnt<float> *> sched_rf;
     std::map<int, HopEnt<double> *> sched_rd;
+    // gather schedule of k_hv_wide: per unit of 64 columns {first entry, slots};
+    // the entries {byte offset of the target column in a plane, signed
+    // coupling} of a slot are [32 lanes][2], columns 64 unit + 2 lane + {0, 1}.
+    // The targets of the 8 lanes of a quarter warp lie in 8 different 16-byte
+    // bank groups.
+    int2 *wide_hdr = nullptr;
+    HopEnt<float> *wide_ent = nullptr;
     int max_cnt = 0;              // largest hop_cnt over words
     int max_group = 0;            // largest bath group (words sharing their bath bits)
     // row items for a given rows-per-item R: whole bath groups packed into
@@ -341,6 +348,8 @@ void hv_fill_job(const mo_ed_ctx *ctx, const Sector &s, int R, const void *x, vo
 // v = tile-shape variant (hv_prepare); all jobs use its rows per item.
 int hv_launch_f32(mo_ed_ctx *ctx, int v, const HvJobT<float> *jobs, int njobs);
 int hv_launch_f64(mo_ed_ctx *ctx, int kind, int v, const HvJobT<double> *jobs, int njobs);
+// R = kWideKey + rows: the packing of k_hv_wide.
+constexpr int kWideKey = 100;
 int species_items(mo_ed_ctx *ctx, Species *sp, int R, const int **items, int *nitems);
 // Tile-shape variant for sector s (autotuned on the first call per shape;
 // that first call allocates and synchronizes, so make it before any stream
@@ -353,6 +362,8 @@ int hv_tuning(mo_ed_ctx *ctx, const Sector &s, int kind, int cap, int *nvar, int
 int hv_prepare_rows(mo_ed_ctx *ctx, const Sector &s, int kind, int v);
 // Per-R stage offsets of the up-spin gather schedule (built once per R).
 int species_sched(mo_ed_ctx *ctx, Species *sp, int R);
+// Gather schedule of k_hv_wide (Species::wide_*), built once.
+int species_wide(mo_ed_ctx *ctx, Species *sp);
 // Down-spin block tables of a species (split H*v), built once; chunk table
 // for row stride ld.
 int species_dblocks(mo_ed_ctx *ctx, Species *sp, int ld);

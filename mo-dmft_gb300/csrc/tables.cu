@@ -63,6 +63,8 @@ Species::~Species()
     cudaFree(dblk_mv_f);
     cudaFree(dblk_mv_d);
     for (auto &kv : dblk_chunks) cudaFree(kv.second);
+    cudaFree(wide_hdr);
+    cudaFree(wide_ent);
 }
 
 // ---------------------------------------------------------------------------
@@ -441,6 +443,38 @@ int species_items(mo_ed_ctx *ctx, Species *sp, int R, const int **items, int *ni
                      [](const Group &a, const Group &b) { return a.key < b.key; });
     std::vector<int> tab;
     int fill = R;
+    if (R >= kWideKey) {
+        // k_hv_wide: every 4 rows are a slot (rows 0-2) for a bath group of 2
+        // or 3 rows, or for single rows, and a single row; groups and single
+        // rows advance together along the sorted order
+        const int rows = R - kWideKey, slots = rows / 4;
+        std::vector<const Group *> multi;
+        std::vector<int> single;
+        int gs = 3;
+        for (const Group &g : groups) {
+            if (g.size > 3) return fail(ctx, MO_ED_ERR_ARG, "bath groups too large for this H*v tile shape");
+            if (g.size > 1) {
+                multi.push_back(&g);
+                gs = g.size;
+            } else {
+                single.push_back(g.first);
+            }
+        }
+        const size_t nm = multi.size(), nsg = single.size();
+        const size_t n = std::max<size_t>({(nm + slots - 1) / slots, (nsg + (size_t)gs * nm + rows - 1) / rows, 1});
+        size_t im = 0, is = 0;
+        for (size_t k = 0; im < nm || is < nsg; ++k) {
+            const bool rest = k + 1 >= n;
+            const size_t last_m = rest ? nm : (k + 1) * nm / n, last_s = rest ? nsg : (k + 1) * nsg / n;
+            std::vector<int> row(rows, -1);
+            for (int slot = 0; slot < slots && im < last_m; ++slot, ++im)
+                for (int i = 0; i < multi[im]->size; ++i) row[4 * slot + i] = multi[im]->first + i;
+            for (int o = rows - 1; o >= 0; --o)
+                if (row[o] < 0 && is < last_s) row[o] = single[is++];
+            tab.insert(tab.end(), row.begin(), row.end());
+        }
+        groups.clear();
+    }
     for (const Group &g : groups) {
         for (int off = 0; off < g.size; off += R) {       // a group larger than R is split
             const int len = std::min(R, g.size - off);
@@ -452,7 +486,7 @@ int species_items(mo_ed_ctx *ctx, Species *sp, int R, const int **items, int *ni
             fill += len;
         }
     }
-    const int n_items = (int)(tab.size() / R);
+    const int n_items = (int)(tab.size() / (R >= kWideKey ? R - kWideKey : R));
     int *d = nullptr;
     MOED_CUDA(ctx, cudaMalloc(&d, sizeof(int) * std::max<size_t>(1, tab.size())));
     MOED_CUDA(ctx, cudaMemcpyAsync(d, tab.data(), sizeof(int) * tab.size(), cudaMemcpyHostToDevice, ctx->stream));
@@ -776,6 +810,87 @@ int species_sched(mo_ed_ctx *ctx, Species *sp, int R)
                                    ctx->stream));
     MOED_CUDA(ctx, cudaMemcpyAsync(dd, ed.data(), sizeof(HopEnt<double>) * ed.size(), cudaMemcpyHostToDevice,
                                    ctx->stream));
+    MOED_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    return MO_ED_OK;
+}
+
+int species_wide(mo_ed_ctx *ctx, Species *sp)
+{
+    if (sp->wide_ent) return MO_ED_OK;
+    const int nunit = (sp->n_pad + 63) / 64;
+    // the moves of every column, from the 32-column schedule
+    std::vector<std::vector<unsigned>> mv(sp->n_pad);
+    for (size_t c = 0; c < sp->h_sched_hdr.size(); ++c)
+        for (int s = 0; s < sp->h_sched_hdr[c].y; ++s)
+            for (int l = 0; l < 32; ++l) {
+                const unsigned e = sp->h_sched_ent[(size_t)sp->h_sched_hdr[c].x + 32 * (size_t)s + l];
+                if (e & 0x80000000u) mv[32 * c + l].push_back(e);
+            }
+    std::vector<int2> hdr(nunit);
+    std::vector<HopEnt<float>> ent;
+    std::vector<int> el[8], eb[8], colour;
+    std::vector<unsigned> code[8];
+    for (int c = 0; c < nunit; ++c) {
+        int delta = 0, dq[8] = {0};        // slots of the unit, and of each quarter
+        for (int pq = 0; pq < 8; ++pq) {   // column parity, quarter warp
+            el[pq].clear();
+            eb[pq].clear();
+            code[pq].clear();
+            int dl[8] = {0}, db[8] = {0};
+            for (int l = 0; l < 8; ++l) {
+                const int u = 64 * c + 2 * (8 * (pq >> 1) + l) + (pq & 1);
+                if (u >= sp->n) continue;
+                for (unsigned e : mv[u]) {
+                    el[pq].push_back(l);
+                    eb[pq].push_back((int)(e & 7u));
+                    code[pq].push_back(e);
+                    dq[pq] = std::max(dq[pq], std::max(++dl[l], ++db[e & 7u]));
+                }
+            }
+            delta = std::max(delta, dq[pq]);
+        }
+        hdr[c] = make_int2((int)ent.size(), delta);
+        const size_t base = ent.size();
+        ent.resize(base + 64 * (size_t)delta);
+        for (int pq = 0; pq < 8; ++pq) {
+            std::vector<unsigned> grid((size_t)8 * delta, 0u);
+            if (!el[pq].empty()) {
+                colour_chunk(el[pq], eb[pq], dq[pq], colour);
+                for (size_t i = 0; i < colour.size(); ++i) {
+                    unsigned &g = grid[(size_t)8 * colour[i] + el[pq][i]];
+                    if (colour[i] < 0 || colour[i] >= dq[pq] || g != 0u)
+                        return fail(ctx, MO_ED_ERR_STATE, "gather schedule colouring failed");
+                    g = code[pq][i];
+                }
+            }
+            for (int s = 0; s < delta; ++s) {
+                unsigned used = 0u;
+                for (int l = 0; l < 8; ++l)
+                    if (grid[8 * s + l]) used |= 1u << (grid[8 * s + l] & 7u);
+                for (int l = 0; l < 8; ++l) {
+                    const unsigned e = grid[8 * s + l];
+                    HopEnt<float> &o = ent[base + 64 * (size_t)s + 2 * (8 * (pq >> 1) + l) + (pq & 1)];
+                    if (e) {
+                        const double v = ctx->cpl_val[(e >> 16) & 63u];
+                        o.t = (int)(e & 0xffffu) * 16;
+                        o.v = (float)((e & (1u << 22)) ? -v : v);
+                    } else {   // a bank group no lane of the quarter reads, coupling 0
+                        const int b = __builtin_ctz(~used);
+                        used |= 1u << b;
+                        o.t = 16 * b;
+                        o.v = 0.0f;
+                    }
+                }
+            }
+        }
+    }
+    if (ent.empty()) ent.resize(1);
+    if (!sp->wide_hdr) MOED_CUDA(ctx, cudaMalloc(&sp->wide_hdr, sizeof(int2) * nunit));
+    HopEnt<float> *d = nullptr;
+    MOED_CUDA(ctx, cudaMalloc(&d, sizeof(HopEnt<float>) * ent.size()));
+    sp->wide_ent = d;
+    MOED_CUDA(ctx, cudaMemcpyAsync(sp->wide_hdr, hdr.data(), sizeof(int2) * nunit, cudaMemcpyHostToDevice, ctx->stream));
+    MOED_CUDA(ctx, cudaMemcpyAsync(d, ent.data(), sizeof(HopEnt<float>) * ent.size(), cudaMemcpyHostToDevice, ctx->stream));
     MOED_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     return MO_ED_OK;
 }

@@ -308,7 +308,8 @@ class EDSolver:
 
     def hv_tuning(self, ne_up, ne_down, dtype=FP32):
         """Autotuner record: list of ((R, threads, CTAs/SM, kernel), ms) and the chosen index;
-        kernel 0 k_hv, 1 k_hv_async, 2 / 3 split (k_hv_down on 128- / 64-byte slices + k_hv_async)."""
+        kernel 0 k_hv / k_hv_row, 1 k_hv_async / k_hv_wide, 2 / 3 split (k_hv_down on 128- / 64-byte slices +
+        k_hv_async), 4 split (k_hv_down_rows + k_hv_async / k_hv_wide)."""
         cap = 16
         nv, ch = C.c_int(), C.c_int()
         shape = np.zeros(4 * cap, np.int32)

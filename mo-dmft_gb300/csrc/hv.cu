@@ -35,6 +35,7 @@
 // k_hv_async (below): double-buffered asynchronous stage, conflict-free
 // scheduled up-spin gathers, precomputed item descriptors.  k_hv_wide: the
 // FP32 successor of it for up to three orbitals.  k_hv_row: small sectors.
+// k_hv_sorted: FP64 sums.
 //
 // Split (below): k_hv_down computes the down-spin hybridisation over
 // down-spin blocks x column slices from shared memory, or k_hv_down_rows as
@@ -47,6 +48,7 @@
 #include <tuple>
 
 #include "internal.h"
+#include "math64.cuh"
 
 namespace moed {
 
@@ -1617,6 +1619,141 @@ k_hv_wide(const __grid_constant__ HvBatch<float> batch, const ModelDev *__restri
     }
 }
 
+// ---------------------------------------------------------------------------
+// k_hv_sorted: FP64 sums (FP64 or FP32 x), one row per CTA.
+// Bound by the FP64 pipe, which a warp instruction holds for 64 cycles
+// whatever its active lanes: k_hv issues a chunk's largest move count for
+// every column of it (57 % of the lanes of 3 orbitals x 4 levels have a move)
+// and FP32 x takes conversions on the same pipe.  Here
+//   * the up-spin moves, the diagonal and the 4-operator terms run over
+//     columns sorted by impurity pattern and move count (species_sorted): the
+//     lanes of a warp have the same number of moves and the same 4-operator
+//     terms;
+//   * their sums go to a second shared-memory row; after one barrier the
+//     down-spin AXPYs, uniform over the row, run in column order and write y;
+//   * FP32 x is widened with integer operations, once per staged element and
+//     per AXPY operand.
+// One row and its sums are 104 KB at most, so two CTAs per SM overlap their
+// loads.  FP64, us: 32 million elements of 3 orbitals x 4 levels 1,646 (k_hv)
+// -> 1,012 (15 FP64 instructions per element take 830 at the pipe's rate),
+// 0.85 million of 3 x 3 61 -> 33, dense V of 2 x 11 (2.9 million) 214 -> 163.
+// ---------------------------------------------------------------------------
+constexpr int kSortTerms = 6;   // 4-operator terms of a (row, pattern): at most (norb / 2)^2
+
+template <typename TX, typename TY, int NT, int MINB>
+__global__ void __launch_bounds__(NT, MINB)
+k_hv_sorted(const __grid_constant__ HvBatch<double> batch, const ModelDev *__restrict__ mdl, int ldmax)
+{
+    constexpr int NW = NT / 32;
+    extern __shared__ __align__(16) double smem_sorted[];
+    double *const S = smem_sorted, *const A = S + ldmax;
+    __shared__ double s_coef[2 * kMaxHop + 1], s_c[kMaxImp], s_jc[kMaxImp][kSortTerms], s_v[kMaxHop], s_red[NW];
+    __shared__ int s_jn[kMaxImp], s_jo[kMaxImp][kSortTerms], s_off[kMaxHop];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int nimp = mdl->nimp, npair = mdl->npair, ncpl = mdl->ncpl;
+    for (int i = tid; i <= 2 * ncpl; i += NT)
+        s_coef[i] = i == 2 * ncpl ? 0.0 : (i & 1) ? -mdl->cval[i >> 1] : mdl->cval[i >> 1];
+
+    for (int cur = hv_next_item(batch, (int)blockIdx.x); cur >= 0; cur = hv_next_item(batch, cur + (int)gridDim.x)) {
+        const HvJobT<double> &jb = batch.job[hv_find_job(batch, cur)];
+        const int it = cur - jb.item0, ld = jb.ld, nd = jb.nd, d = __ldg(jb.items + it);
+        const TX *__restrict__ x = (const TX *)jb.x;
+        const TX *__restrict__ xd = x + (size_t)d * ld;
+        TY *__restrict__ y = (TY *)jb.y + (size_t)d * ld;
+        const int dinf = __ldg(jb.dn_info + d), id = (dinf >> 8) & 0xff, cnt = dinf & 0xff;
+        __syncthreads();   // the previous row is done with shared memory
+        for (int i = tid; i < cnt; i += NT) {
+            s_off[i] = __ldg(jb.dn_tgt + (size_t)i * nd + d) * ld;
+            s_v[i] = __ldg(jb.dn_val + (size_t)i * nd + d);
+        }
+        for (int iu = tid; iu < nimp; iu += NT) {
+            s_c[iu] = mdl->cross[iu * nimp + id] + __ldg(jb.dn_diag + d);
+            // spin-flip and pair-hop terms of this row for columns of pattern iu
+            int n = 0;
+            for (int p = 0; p < npair; ++p) {
+                const int e = mdl->t4[p * nimp + iu];
+                if (e >= 0) continue;
+                const int esf = mdl->t4[mdl->pair_rev[p] * nimp + id], eph = mdl->t4[p * nimp + id];
+                const int f = esf < 0 ? esf : eph;   // T_{j<-i}(d) or T_{i<-j}(d): never both
+                if (f < 0 && n < kSortTerms) {
+                    s_jo[iu][n] = (d + (int)(short)(f & 0xffff)) * ld + (int)(short)(e & 0xffff);
+                    s_jc[iu][n] = ((e ^ f) & 0x40000000) ? -mdl->J : mdl->J;
+                    ++n;
+                }
+            }
+            s_jn[iu] = n;
+        }
+        for (int u = tid; u < ld; u += NT) {
+            S[u] = widen(__ldg(xd + u));
+            if (u >= jb.nu) A[u] = 0.0;
+        }
+        __syncthreads();
+        for (int c = warp; c < jb.srt_n; c += NW) {
+            const int2 h = __ldg(jb.srt_hdr + c);
+            const int uc = __ldg(jb.srt_col + 32 * c + lane), u = max(uc, 0);
+            const int ns = h.y & 0xffff, iu = h.y >> 16;
+            const unsigned *ent = jb.srt_ent + h.x + lane;
+            // the loops below end by a branch: a predicated-off FP64 instruction
+            // would hold the pipe as long as one that counts.  The operands
+            // of the next QE / QD turns are in flight in a queue.
+            constexpr int QE = 4;
+            unsigned e[QE];
+#pragma unroll
+            for (int t = 0; t < QE; ++t) e[t] = t < ns ? __ldg(ent + 32 * t) : 0u;
+            const int nj = s_jn[iu];
+            double acc = (__ldg(jb.up_diag + u) + s_c[iu]) * S[u];
+            if (nj > 0) {
+                TX g = __ldg(x + (s_jo[iu][0] + u));
+#pragma unroll 1
+                for (int t = 0; t < nj; ++t) {
+                    const TX h2 = t + 1 < nj ? __ldg(x + (s_jo[iu][t + 1] + u)) : TX(0);
+                    acc = fma(s_jc[iu][t], widen(g), acc);
+                    g = h2;
+                }
+            }
+#pragma unroll 1
+            for (int s = 0; s < ns; ++s) {
+                const unsigned m = e[0];
+#pragma unroll
+                for (int t = 0; t + 1 < QE; ++t) e[t] = e[t + 1];
+                e[QE - 1] = s + QE < ns ? __ldg(ent + 32 * (s + QE)) : 0u;
+                acc = fma(s_coef[m >> 16], S[m & 0xffffu], acc);
+            }
+            if (uc >= 0) A[u] = acc;
+        }
+        __syncthreads();
+        const bool want_dot = jb.dot_partial != nullptr;
+        double dacc = 0.0;
+        for (int u = tid; u < ld; u += NT) {   // ld is a multiple of 32: whole warps
+            double acc = A[u];
+            constexpr int QD = 6;
+            TX g[QD];
+#pragma unroll
+            for (int t = 0; t < QD; ++t) g[t] = t < cnt ? __ldg(x + (s_off[t] + u)) : TX(0);
+#pragma unroll 1
+            for (int s = 0; s < cnt; ++s) {
+                const TX h2 = g[0];
+#pragma unroll
+                for (int t = 0; t + 1 < QD; ++t) g[t] = g[t + 1];
+                g[QD - 1] = s + QD < cnt ? __ldg(x + (s_off[s + QD] + u)) : TX(0);
+                acc = fma(s_v[s], widen(h2), acc);
+            }
+            y[u] = (TY)acc;
+            if (want_dot) dacc = fma(S[u], acc, dacc);
+        }
+        if (want_dot) {
+            for (int off = 16; off > 0; off >>= 1) dacc += __shfl_down_sync(0xffffffffu, dacc, off);
+            if (lane == 0) s_red[warp] = dacc;
+            __syncthreads();
+            if (tid == 0) {
+                double t = 0.0;
+                for (int w = 0; w < NW; ++w) t += s_red[w];
+                jb.dot_partial[it] = t;
+            }
+        }
+    }
+}
+
 template <typename TX, typename TA, int R>
 static size_t dyn_smem_bytes_async(int ld, const ModelDev &m, const DescGeom &g)
 {
@@ -1641,16 +1778,18 @@ struct HvVariant {
     // 4: split, k_hv_down_rows (row AXPYs from L2) + k_hv_async<SPLIT>
     int staged;
     bool wide = false;   // k_hv_wide in the place of k_hv_async
+    bool sorted = false; // k_hv_sorted (one row per item)
     int key() const { return wide ? kWideKey + R : R; }   // of the item table
 };
 static const HvVariant kVarF32[] = {{4, 512, 2, 1, true}, {4, 256, 2, 0}, {6, 512, 1, 0}, {3, 256, 3, 0},
                                     {8, 832, 1, 4, true}, {4, 512, 1, 1}, {3, 512, 1, 1}, {4, 512, 2, 4, true},
                                     {2, 256, 2, 1}, {3, 512, 1, 2}, {4, 512, 1, 2}, {3, 512, 1, 3},
                                     {3, 512, 1, 4}, {4, 512, 1, 4}, {4, 512, 1, 4}, {1, 128, 8, 0}};
-static const HvVariant kVarF64[] = {{2, 256, 2, 0}, {3, 256, 1, 0}, {2, 512, 1, 0}, {2, 512, 1, 1},
-                                    {4, 512, 1, 1}, {2, 512, 1, 2}, {2, 512, 1, 3}, {2, 512, 1, 4}, {1, 128, 8, 0}};
-static const int kRowVarF32 = 15, kRowVarF64 = 8;   // k_hv_row
-static const int kSmallVarF32 = 8;                   // k_hv_async<2, 256>: two CTAs per SM
+static const HvVariant kVarF64[] = {{2, 512, 1, 1}, {2, 512, 1, 2}, {2, 512, 1, 4}, {1, 128, 8, 0},
+                                    {1, 512, 2, 0, false, true}, {1, 256, 4, 0, false, true}, {1, 128, 6, 0, false, true}};
+// the small sectors' shapes (hv_prepare)
+static const int kRowVarF32 = 15, kRowVarF64 = 3;       // k_hv_row
+static const int kSmallVarF32 = 8, kSmallVarF64 = 5;    // k_hv_async<2, 256>, k_hv_sorted<256>
 static const int kNVarF32 = sizeof(kVarF32) / sizeof(kVarF32[0]);
 static const int kNVarF64 = sizeof(kVarF64) / sizeof(kVarF64[0]);
 
@@ -1694,6 +1833,10 @@ void hv_fill_job(const mo_ed_ctx *ctx, const Sector &s, int R, const void *x, vo
         auto dsc = s.dn->desc.find(R * 2 + (f32 ? 0 : 1));
         j.desc = dsc != s.dn->desc.end() ? dsc->second : nullptr;
     }
+    j.srt_hdr = s.up->srt_hdr;
+    j.srt_col = s.up->srt_col;
+    j.srt_ent = s.up->srt_ent;
+    j.srt_n = s.up->srt_n;
     j.dblk_off = s.dn->dblk_off;
     j.dblk_rows = s.dn->dblk_rows;
     j.dblk_ptr = s.dn->dblk_ptr;
@@ -1908,6 +2051,25 @@ static int launch_batch_row(mo_ed_ctx *ctx, const HvBatch<TA> &b)
     return MO_ED_OK;
 }
 
+template <typename TX, typename TY, int NT, int MINB>
+static int launch_batch_sorted(mo_ed_ctx *ctx, const HvBatch<double> &b)
+{
+    if (b.total_items <= 0) return MO_ED_OK;
+    int ldmax = 0;
+    for (int i = 0; i < b.njobs; ++i) {
+        ldmax = std::max(ldmax, b.job[i].ld);
+        if (!b.job[i].items || !b.job[i].srt_ent) return fail(ctx, MO_ED_ERR_STATE, "H*v tables missing");
+    }
+    const size_t smem = 2 * sizeof(double) * (size_t)ldmax;
+    auto kern = k_hv_sorted<TX, TY, NT, MINB>;
+    int per_sm = 0;
+    if (int rc = kernel_fit(ctx, kern, NT, smem, &per_sm)) return rc;
+    if (per_sm < 1) return fail(ctx, MO_ED_ERR_ARG, "sector rows too long for the shared-memory stage");
+    kern<<<std::min(b.total_items, ctx->num_sms * per_sm), NT, smem, ctx->stream>>>(b, ctx->d_mdl, ldmax);
+    MOED_CHECK_LAUNCH(ctx);
+    return MO_ED_OK;
+}
+
 // shared memory of k_hv_wide for rows of up to ldmax columns
 static WideLayout wide_layout(int ldmax, int rows, const ModelDev &m, size_t *total)
 {
@@ -2014,27 +2176,23 @@ static int launch_variant(mo_ed_ctx *ctx, int kind, int v, const HvBatch<TA> &b)
         }
     } else if (kind == HV_F64) {
         switch (v) {
-        case 0: return launch_batch<double, double, double, 2, 256, 2>(ctx, b);
-        case 1: return launch_batch<double, double, double, 3, 256, 1>(ctx, b);
-        case 2: return launch_batch<double, double, double, 2, 512, 1>(ctx, b);
-        case 3: return launch_batch_async<double, double, double, 2, 512>(ctx, b);
-        case 4: return launch_batch_async<double, double, double, 4, 512>(ctx, b);
-        case 5: return launch_batch_split<double, double, double, 2, 512, 1, 128>(ctx, b);
-        case 6: return launch_batch_split<double, double, double, 2, 512, 1, 64>(ctx, b);
-        case 7: return launch_batch_rows<double, double, double, 2, 512, 1>(ctx, b);
-        default: return launch_batch_row<double, double, double>(ctx, b);
+        case 0: return launch_batch_async<double, double, double, 2, 512>(ctx, b);
+        case 1: return launch_batch_split<double, double, double, 2, 512, 1, 128>(ctx, b);
+        case 2: return launch_batch_rows<double, double, double, 2, 512, 1>(ctx, b);
+        case 3: return launch_batch_row<double, double, double>(ctx, b);
+        case 4: return launch_batch_sorted<double, double, 512, 2>(ctx, b);
+        case 5: return launch_batch_sorted<double, double, 256, 4>(ctx, b);
+        default: return launch_batch_sorted<double, double, 128, 6>(ctx, b);
         }
     } else {
         switch (v) {
-        case 0: return launch_batch<float, double, double, 2, 256, 2>(ctx, b);
-        case 1: return launch_batch<float, double, double, 3, 256, 1>(ctx, b);
-        case 2: return launch_batch<float, double, double, 2, 512, 1>(ctx, b);
-        case 3: return launch_batch_async<float, double, double, 2, 512>(ctx, b);
-        case 4: return launch_batch_async<float, double, double, 4, 512>(ctx, b);
-        case 5: return launch_batch_split<float, double, double, 2, 512, 1, 128>(ctx, b);
-        case 6: return launch_batch_split<float, double, double, 2, 512, 1, 64>(ctx, b);
-        case 7: return launch_batch_rows<float, double, double, 2, 512, 1>(ctx, b);
-        default: return launch_batch_row<float, double, double>(ctx, b);
+        case 0: return launch_batch_async<float, double, double, 2, 512>(ctx, b);
+        case 1: return launch_batch_split<float, double, double, 2, 512, 1, 128>(ctx, b);
+        case 2: return launch_batch_rows<float, double, double, 2, 512, 1>(ctx, b);
+        case 3: return launch_batch_row<float, double, double>(ctx, b);
+        case 4: return launch_batch_sorted<float, double, 512, 2>(ctx, b);
+        case 5: return launch_batch_sorted<float, double, 256, 4>(ctx, b);
+        default: return launch_batch_sorted<float, double, 128, 6>(ctx, b);
         }
     }
 }
@@ -2090,6 +2248,7 @@ static int prepare_variant(mo_ed_ctx *ctx, const Sector &s, int kind, int v)
     const int *items;
     int n;
     if (int rc = species_items(ctx, s.dn, h.key(), &items, &n)) return rc;
+    if (h.sorted) return species_sorted(ctx, s.up);
     if (!h.staged) return MO_ED_OK;
     if (h.wide) return species_wide(ctx, s.up);
     if (h.staged == 2 || h.staged == 3) {
@@ -2161,10 +2320,12 @@ int hv_prepare(mo_ed_ctx *ctx, const Sector &s, int kind, int *v_out, int *R_out
         v = it->second;
     } else if (s.Dpad() < kTuneMinElems) {
         // small sector: timing the variants would cost more than it saves.
-        // k_hv_row against the best staged variant, us: FP32 8.3 : 8.3 at
-        // 15,876 elements, 10.3 : 8.3 at 63,504, 22.9 : 14.5 at 213,444; FP64
-        // 7.4 : 9.1 at 4,900, 12.4 : 12.4 at 63,504, 34.9 : 37.1 at 213,444.
-        v = kind != HV_F32 ? kRowVarF64 : s.D() < (1 << 15) ? kRowVarF32 : kSmallVarF32;
+        // k_hv_row against the best other shape, us: FP32 (k_hv_async<2, 256>)
+        // 8.3 : 8.3 at 15,876 elements, 10.3 : 8.3 at 63,504, 22.9 : 14.5 at
+        // 213,444; FP64 (k_hv_sorted<256>) 12.4 : 8.3 at 63,504, 34.9 : 24.8 at
+        // 213,444; at 4,900 both are the launch.
+        const bool tiny = s.D() < (1 << 15);
+        v = kind == HV_F32 ? (tiny ? kRowVarF32 : kSmallVarF32) : (tiny ? kRowVarF64 : kSmallVarF64);
         ctx->hv_choice[key] = v;
         ctx->hv_times[key].assign(nvariants(kind), -1.0f);
     } else {
@@ -2210,7 +2371,9 @@ int hv_lookup(mo_ed_ctx *ctx, const Sector &s, int kind, int *v_out, int *R_out)
     const HvVariant &h = variant(kind, it->second);
     const int R = h.key();
     bool ready = s.dn->items.count(R) != 0;
-    if (h.wide)
+    if (h.sorted)
+        ready = ready && s.up->srt_ent != nullptr;
+    else if (h.wide)
         ready = ready && s.up->wide_ent != nullptr;
     else if (h.staged)
         ready = ready && s.up->sched_rf.count(R) && s.dn->desc.count(R * 2 + (kind == HV_F32 ? 0 : 1));

@@ -112,6 +112,14 @@ struct Species {
     // bank groups.
     int2 *wide_hdr = nullptr;
     HopEnt<float> *wide_ent = nullptr;
+    // columns of k_hv_sorted: chunks of 32 columns with one impurity pattern
+    // and nearly one move count.  srt_hdr[chunk] = {first entry, slots |
+    // pattern << 16}, srt_col[32 chunk + lane] the column (-1: none), entry
+    // (slot, lane) = target column | (2 coupling + sign) << 16 (2 ncpl: none)
+    int2 *srt_hdr = nullptr;
+    int *srt_col = nullptr;
+    unsigned *srt_ent = nullptr;
+    int srt_n = 0;                // chunks
     int max_cnt = 0;              // largest hop_cnt over words
     int max_group = 0;            // largest bath group (words sharing their bath bits)
     // row items for a given rows-per-item R: whole bath groups packed into
@@ -171,6 +179,10 @@ struct HvJobT {
     const unsigned *up_sched_ent;
     const HopEnt<TA> *up_sched;
     const unsigned *desc;          // per-item descriptors (staged kernel)
+    const int2 *srt_hdr;           // sorted columns (Species::srt_*)
+    const int *srt_col;
+    const unsigned *srt_ent;
+    int srt_n;
     // down-spin blocks of the split kernel (Species::dblk_*)
     const int *dblk_off, *dblk_rows, *dblk_ptr;
     const HopEnt<TA> *dblk_mv;
@@ -364,6 +376,8 @@ int hv_prepare_rows(mo_ed_ctx *ctx, const Sector &s, int kind, int v);
 int species_sched(mo_ed_ctx *ctx, Species *sp, int R);
 // Gather schedule of k_hv_wide (Species::wide_*), built once.
 int species_wide(mo_ed_ctx *ctx, Species *sp);
+// Sorted columns of k_hv_sorted (Species::srt_*), built once.
+int species_sorted(mo_ed_ctx *ctx, Species *sp);
 // Down-spin block tables of a species (split H*v), built once; chunk table
 // for row stride ld.
 int species_dblocks(mo_ed_ctx *ctx, Species *sp, int ld);

@@ -33,14 +33,20 @@ __device__ __forceinline__ double rcp_pos(double d)
     return fma(y0, fma(e, e, e), y0);
 }
 
-// (double)f by integer operations (a conversion instruction would take a slot
-// of the FP64 pipe); denormals, infinities and NaN take the conversion.
+// (double)f by integer operations: a conversion instruction takes a slot of
+// the FP64 pipe, even one that is predicated off, so the rare cases have none
+// either.  Infinities and NaN need the exponent 2047 instead of 255 + 896; a
+// denormal is scaled by 2^24 in FP32 first.
 __device__ __forceinline__ double widen(float f)
 {
     const unsigned b = __float_as_uint(f);
-    if ((b << 1) == 0u) return __hiloint2double((int)b, 0);
-    if (((b & 0x7f800000u) - 0x00800000u) >= 0x7f000000u) return (double)f;
-    return __hiloint2double((int)((((b & 0x7fffffffu) >> 3) + 0x38000000u) | (b & 0x80000000u)), (int)(b << 29));
+    unsigned m = b & 0x7fffffffu, e = 0x38000000u;   // 896 more in the exponent
+    if (m >= 0x7f800000u) e = 0x70000000u;
+    if (m < 0x00800000u) {
+        m = __float_as_uint(f * 16777216.0f) & 0x7fffffffu;
+        e = m ? 0x38000000u - (24u << 20) : 0u;
+    }
+    return __hiloint2double((int)(((m >> 3) + e) | (b & 0x80000000u)), (int)(m << 29));
 }
 __device__ __forceinline__ double widen(double f) { return f; }
 

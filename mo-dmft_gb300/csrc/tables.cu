@@ -65,6 +65,9 @@ Species::~Species()
     for (auto &kv : dblk_chunks) cudaFree(kv.second);
     cudaFree(wide_hdr);
     cudaFree(wide_ent);
+    cudaFree(srt_hdr);
+    cudaFree(srt_col);
+    cudaFree(srt_ent);
 }
 
 // ---------------------------------------------------------------------------
@@ -814,11 +817,9 @@ int species_sched(mo_ed_ctx *ctx, Species *sp, int R)
     return MO_ED_OK;
 }
 
-int species_wide(mo_ed_ctx *ctx, Species *sp)
+// the moves of every column, from the 32-column schedule
+static std::vector<std::vector<unsigned>> column_moves(const Species *sp)
 {
-    if (sp->wide_ent) return MO_ED_OK;
-    const int nunit = (sp->n_pad + 63) / 64;
-    // the moves of every column, from the 32-column schedule
     std::vector<std::vector<unsigned>> mv(sp->n_pad);
     for (size_t c = 0; c < sp->h_sched_hdr.size(); ++c)
         for (int s = 0; s < sp->h_sched_hdr[c].y; ++s)
@@ -826,6 +827,61 @@ int species_wide(mo_ed_ctx *ctx, Species *sp)
                 const unsigned e = sp->h_sched_ent[(size_t)sp->h_sched_hdr[c].x + 32 * (size_t)s + l];
                 if (e & 0x80000000u) mv[32 * c + l].push_back(e);
             }
+    return mv;
+}
+
+int species_sorted(mo_ed_ctx *ctx, Species *sp)
+{
+    if (sp->srt_ent) return MO_ED_OK;
+    const std::vector<std::vector<unsigned>> mv = column_moves(sp);
+    const int nimp = ctx->mdl.nimp;
+    const unsigned none = 2u * (unsigned)ctx->mdl.ncpl;
+    // columns by impurity pattern, most moves first
+    std::vector<std::vector<int>> by(nimp);
+    int u = 0;
+    for (unsigned w = 0; w < (1u << sp->nsite); ++w)
+        if (__builtin_popcount(w) == sp->N) by[w & (unsigned)(nimp - 1)].push_back(u++);
+    std::vector<int2> hdr;
+    std::vector<int> col;
+    std::vector<unsigned> ent;
+    for (int iu = 0; iu < nimp; ++iu) {
+        std::vector<int> &v = by[iu];
+        std::stable_sort(v.begin(), v.end(), [&](int a, int b) { return mv[a].size() > mv[b].size(); });
+        for (size_t i = 0; i < v.size(); i += 32) {
+            const int slots = (int)mv[v[i]].size();
+            hdr.push_back(make_int2((int)ent.size(), slots | iu << 16));
+            const size_t base = ent.size();
+            ent.resize(base + 32 * (size_t)slots, none << 16);
+            for (int l = 0; l < 32; ++l) {
+                const bool live = i + l < v.size();
+                col.push_back(live ? v[i + l] : -1);
+                if (!live) continue;
+                for (size_t s = 0; s < mv[v[i + l]].size(); ++s) {
+                    const unsigned e = mv[v[i + l]][s];
+                    ent[base + 32 * s + l] = (e & 0xffffu) | ((2u * ((e >> 16) & 63u) + ((e >> 22) & 1u)) << 16);
+                }
+            }
+        }
+    }
+    if (ent.empty()) ent.push_back(none << 16);
+    if (!sp->srt_hdr) MOED_CUDA(ctx, cudaMalloc(&sp->srt_hdr, sizeof(int2) * hdr.size()));
+    if (!sp->srt_col) MOED_CUDA(ctx, cudaMalloc(&sp->srt_col, sizeof(int) * col.size()));
+    unsigned *d = nullptr;
+    MOED_CUDA(ctx, cudaMalloc(&d, sizeof(unsigned) * ent.size()));
+    sp->srt_ent = d;
+    sp->srt_n = (int)hdr.size();
+    MOED_CUDA(ctx, cudaMemcpyAsync(sp->srt_hdr, hdr.data(), sizeof(int2) * hdr.size(), cudaMemcpyHostToDevice, ctx->stream));
+    MOED_CUDA(ctx, cudaMemcpyAsync(sp->srt_col, col.data(), sizeof(int) * col.size(), cudaMemcpyHostToDevice, ctx->stream));
+    MOED_CUDA(ctx, cudaMemcpyAsync(d, ent.data(), sizeof(unsigned) * ent.size(), cudaMemcpyHostToDevice, ctx->stream));
+    MOED_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    return MO_ED_OK;
+}
+
+int species_wide(mo_ed_ctx *ctx, Species *sp)
+{
+    if (sp->wide_ent) return MO_ED_OK;
+    const int nunit = (sp->n_pad + 63) / 64;
+    const std::vector<std::vector<unsigned>> mv = column_moves(sp);
     std::vector<int2> hdr(nunit);
     std::vector<HopEnt<float>> ent;
     std::vector<int> el[8], eb[8], colour;

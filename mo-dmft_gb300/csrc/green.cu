@@ -495,12 +495,14 @@ int calc_green(mo_ed_ctx *ctx, double *Gr)
         std::vector<int> nc;
         if (int rc = lz_run(ctx, lb, a, bb, nc)) return rc;
         // normsq = ||start||^2 (ed_green.F90:157): nrm[0] of each run
-        std::vector<double> coef(lb.coef.bytes / sizeof(double));
-        MOED_CUDA(ctx, cudaMemcpyAsync(coef.data(), lb.coef.p, lb.coef.bytes, cudaMemcpyDeviceToHost, ctx->stream));
+        const size_t per = (size_t)4 * (nstep + 1);
+        std::vector<double> coef(per * (b1 - b0));
+        MOED_CUDA(ctx, cudaMemcpyAsync(coef.data(), lb.coef, sizeof(double) * coef.size(), cudaMemcpyDeviceToHost,
+                                       ctx->stream));
         MOED_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
         for (size_t k = b0; k < b1; ++k) {
             const int r = (int)(k - b0), i = valid[k];
-            normsq[i] = coef[(size_t)2 * (nstep + 1) * r + (nstep + 1)];
+            normsq[i] = coef[per * r + (nstep + 1)];
             nsc[i] = nc[r];
             A[i] = a[r];
             B[i] = bb[r];

@@ -194,6 +194,8 @@ struct HvJobT {
 // ---------------------------------------------------------------------------
 // context
 // ---------------------------------------------------------------------------
+constexpr size_t kLzPoolBytes = (size_t)512 << 20;
+
 struct DevBuf {              // owning device allocation (move-only)
     void *p = nullptr;
     size_t bytes = 0;
@@ -296,6 +298,7 @@ struct mo_ed_ctx {
     // kKryPoolBytes together), small arrays, and pinned host memory for the
     // coefficients read while the next steps run
     std::vector<moed::DevBuf> kry_pool, kry_small;
+    moed::DevBuf lz_pool;      // workspace of lanczos_iteration and the Green's function, up to kLzPoolBytes
     void *pinned = nullptr;
     size_t pinned_bytes = 0;
     // autotuned H*v tile shape per (kind, Nup, Ndn), and the timings (ms) of

@@ -94,7 +94,7 @@ __global__ void k_lz_norm0(const __grid_constant__ LzBatchDev b)
         const int r = find_run_upd(b, item);
         const LzRunDev &R = b.run[r];
         const int it = item - R.upd_item0;
-        const long long i0 = (long long)it * kVecChunk, i1 = min(R.D, i0 + kVecChunk);
+        const long long i0 = (long long)it * R.chunk, i1 = min(R.D, i0 + R.chunk);
         const T *u = (const T *)R.u[0];
         double acc = 0.0;
         for (long long i = i0 + threadIdx.x; i < i1; i += blockDim.x) acc += (double)u[i] * (double)u[i];
@@ -112,23 +112,13 @@ template <typename T>
 __global__ void k_lz_update(const __grid_constant__ LzBatchDev b, int j)
 {
     __shared__ double sred[32];
-    __shared__ T coef[3];
     for (int item = blockIdx.x; item < b.total_items; item += gridDim.x) {
         const int r = find_run_upd(b, item);
         const LzRunDev &R = b.run[r];
         if (*R.active == 0) continue;
         const int it = item - R.upd_item0;
-        const long long i0 = (long long)it * kVecChunk, i1 = min(R.D, i0 + kVecChunk);
-        // square roots and divisions are tens of FP64 instructions: one thread's
-        __syncthreads();   // the previous item has read coef
-        if (threadIdx.x == 0) {
-            const double nb1 = R.nrm[j - 1];
-            coef[0] = (T)(1.0 / sqrt(nb1));
-            coef[1] = (T)R.a[j - 1];
-            coef[2] = (j >= 2) ? (T)sqrt(nb1 / R.nrm[j - 2]) : T(0);
-        }
-        __syncthreads();
-        const T s = coef[0], a = coef[1], c = coef[2];
+        const long long i0 = (long long)it * R.chunk, i1 = min(R.D, i0 + R.chunk);
+        const T s = (T)R.inv[j - 1], a = (T)R.a[j - 1], c = (j >= 2) ? (T)R.cpl[j - 1] : T(0);
         const T *w = (const T *)R.w;
         const T *uc = (const T *)R.u[(j - 1) % 3];
         const T *up = (const T *)R.u[(j + 1) % 3];   // (j-2) mod 3
@@ -186,6 +176,10 @@ __global__ void k_lz_finalize(const __grid_constant__ LzBatchDev b, int j, int n
             return;
         }
         R.a[j] = dot / nrm;
+        // for the next update: square roots and divisions are tens of FP64
+        // instructions, so not in its threads
+        R.inv[j] = 1.0 / sqrt(nrm);
+        R.cpl[j] = j > 0 ? sqrt(nrm / R.nrm[j - 1]) : 0.0;
         const double tiny = (double)1.e-12f;
         if (j >= 1 && nrm < tiny) {
             *R.nstep_calc = j;
@@ -197,7 +191,9 @@ __global__ void k_lz_finalize(const __grid_constant__ LzBatchDev b, int j, int n
     }
 }
 
-void *lz_start_vector(LzBatch &b, int r) { return b.vecs[4 * r].p; }
+void *lz_start_vector(LzBatch &b, int r) { return b.vecs[4 * r]; }
+
+static size_t up256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 int lz_setup(mo_ed_ctx *ctx, LzBatch &b, const std::vector<Sector> &secs, int prec, int nstep)
 {
@@ -206,22 +202,6 @@ int lz_setup(mo_ed_ctx *ctx, LzBatch &b, const std::vector<Sector> &secs, int pr
     b.prec = prec;
     b.nstep = nstep;
     b.sec = secs;
-    b.vecs.clear();
-    b.vecs.resize(4 * nrun);
-    const size_t es = prec == MO_ED_FP32 ? sizeof(float) : sizeof(double);
-    for (int r = 0; r < nrun; ++r)
-        for (int k = 0; k < 4; ++k)
-            if (int rc = dev_alloc(ctx, b.vecs[4 * r + k], es * (size_t)secs[r].Dpad())) return rc;
-    if (int rc = dev_alloc(ctx, b.coef, sizeof(double) * 2 * (nstep + 1) * nrun)) return rc;
-    if (int rc = dev_alloc(ctx, b.flags, sizeof(int) * 2 * nrun)) return rc;
-    MOED_CUDA(ctx, cudaMemsetAsync(b.coef.p, 0, b.coef.bytes, ctx->stream));
-    std::vector<int> fl(2 * nrun);
-    for (int r = 0; r < nrun; ++r) {
-        fl[2 * r] = 1;
-        fl[2 * r + 1] = 0;
-    }
-    MOED_CUDA(ctx, cudaMemcpyAsync(b.flags.p, fl.data(), sizeof(int) * 2 * nrun,
-                                   cudaMemcpyHostToDevice, ctx->stream));
     b.upd_item0.resize(nrun);
     b.upd_nitems.resize(nrun);
     b.hv_item0.resize(nrun);
@@ -233,17 +213,46 @@ int lz_setup(mo_ed_ctx *ctx, LzBatch &b, const std::vector<Sector> &secs, int pr
     for (int r = 1; r < nrun; ++r)
         if (secs[r].D() > secs[big].D()) big = r;
     if (int rc = hv_prepare(ctx, secs[big], kind, &b.hv_variant, &b.hv_rows)) return rc;
+    const size_t es = prec == MO_ED_FP32 ? sizeof(float) : sizeof(double);
+    size_t vbytes = 0;
     for (int r = 0; r < nrun; ++r) {
         if (int rc = hv_prepare_rows(ctx, secs[r], kind, b.hv_variant)) return rc;
+        const int chunk = vec_chunk(secs[r].Dpad());
         b.upd_item0[r] = b.upd_total;
-        b.upd_nitems[r] = (int)((secs[r].Dpad() + kVecChunk - 1) / kVecChunk);
+        b.upd_nitems[r] = (int)((secs[r].Dpad() + chunk - 1) / chunk);
         b.upd_total += b.upd_nitems[r];
         b.hv_item0[r] = b.hv_total;
         b.hv_nitems[r] = secs[r].dn->nitems.at(b.hv_rows);
         b.hv_total += b.hv_nitems[r];
+        vbytes += 4 * up256(es * (size_t)secs[r].Dpad());
     }
-    if (int rc = dev_alloc(ctx, b.upd_part, sizeof(double) * std::max(1, b.upd_total))) return rc;
-    if (int rc = dev_alloc(ctx, b.hv_part, sizeof(double) * std::max(1, b.hv_total))) return rc;
+    // one workspace: kept in the context up to kLzPoolBytes (an allocation
+    // costs more than several steps of a small sector)
+    const size_t ncoef = (size_t)4 * (nstep + 1) * nrun;
+    const size_t ocoef = vbytes, oflags = ocoef + up256(sizeof(double) * ncoef), oupd = oflags + up256(sizeof(int) * 2 * nrun);
+    const size_t ohv = oupd + up256(sizeof(double) * std::max(1, b.upd_total));
+    const size_t total = ohv + up256(sizeof(double) * std::max(1, b.hv_total));
+    DevBuf &ws = total <= kLzPoolBytes ? ctx->lz_pool : b.own;
+    if (int rc = ensure(ctx, ws, total)) return rc;
+    char *base = (char *)ws.p;
+    b.vecs.clear();
+    size_t o = 0;
+    for (int r = 0; r < nrun; ++r)
+        for (int k = 0; k < 4; ++k) {
+            b.vecs.push_back(base + o);
+            o += up256(es * (size_t)secs[r].Dpad());
+        }
+    b.coef = (double *)(base + ocoef);
+    b.flags = (int *)(base + oflags);
+    b.upd_part = (double *)(base + oupd);
+    b.hv_part = (double *)(base + ohv);
+    MOED_CUDA(ctx, cudaMemsetAsync(b.coef, 0, sizeof(double) * ncoef, ctx->stream));
+    std::vector<int> fl(2 * nrun);
+    for (int r = 0; r < nrun; ++r) {
+        fl[2 * r] = 1;
+        fl[2 * r + 1] = 0;
+    }
+    MOED_CUDA(ctx, cudaMemcpyAsync(b.flags, fl.data(), sizeof(int) * 2 * nrun, cudaMemcpyHostToDevice, ctx->stream));
     return MO_ED_OK;
 }
 
@@ -253,28 +262,34 @@ static void lz_fill_dev(LzBatch &b, LzBatchDev &d)
     memset(&d, 0, sizeof(d));
     d.nrun = nrun;
     d.total_items = b.upd_total;
-    double *coef = (double *)b.coef.p;
-    int *fl = (int *)b.flags.p;
     for (int r = 0; r < nrun; ++r) {
         LzRunDev &R = d.run[r];
-        for (int k = 0; k < 3; ++k) R.u[k] = b.vecs[4 * r + k].p;
-        R.w = b.vecs[4 * r + 3].p;
+        for (int k = 0; k < 3; ++k) R.u[k] = b.vecs[4 * r + k];
+        R.w = b.vecs[4 * r + 3];
         R.D = b.sec[r].Dpad();
+        R.chunk = vec_chunk(R.D);
         R.upd_item0 = b.upd_item0[r];
         R.upd_nitems = b.upd_nitems[r];
         R.hv_item0 = b.hv_item0[r];
         R.hv_nitems = b.hv_nitems[r];
-        R.a = coef + (size_t)2 * (b.nstep + 1) * r;
+        R.a = b.coef + (size_t)4 * (b.nstep + 1) * r;
         R.nrm = R.a + (b.nstep + 1);
-        R.active = fl + 2 * r;
-        R.nstep_calc = fl + 2 * r + 1;
-        R.upd_part = (double *)b.upd_part.p + b.upd_item0[r];
-        R.hv_part = (double *)b.hv_part.p + b.hv_item0[r];
+        R.inv = R.nrm + (b.nstep + 1);
+        R.cpl = R.inv + (b.nstep + 1);
+        R.active = b.flags + 2 * r;
+        R.nstep_calc = b.flags + 2 * r + 1;
+        R.upd_part = b.upd_part + b.upd_item0[r];
+        R.hv_part = b.hv_part + b.hv_item0[r];
     }
 }
 
+// All nstep+1 steps of a batch: 3 launches per step (4 with a split H*v), no
+// host round trip (runs stop on the device through their active flags).  The
+// launches go out faster than the kernels run, so a graph of them, used once,
+// only adds its instantiation (50 FP64 steps of 0.73 million elements: 0.6 ms
+// of 5.1 ms).
 template <typename T>
-static int lz_enqueue(mo_ed_ctx *ctx, LzBatch &b, LzBatchDev &d)
+static int lz_steps(mo_ed_ctx *ctx, LzBatch &b, LzBatchDev &d)
 {
     const int nrun = d.nrun;
     const int kind = sizeof(T) == 4 ? HV_F32 : HV_F64;
@@ -305,56 +320,26 @@ static int lz_enqueue(mo_ed_ctx *ctx, LzBatch &b, LzBatchDev &d)
     return MO_ED_OK;
 }
 
-// All nstep+1 steps of a batch (3 launches per step, no host round trip:
-// runs stop on the device through their active flags).  With `graph` the
-// launches are captured once into a CUDA graph and replayed as one launch;
-// a stream that is already being captured gets the plain launches.
-template <typename T>
-static int lz_steps(mo_ed_ctx *ctx, LzBatch &b, LzBatchDev &d, bool graph)
-{
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    MOED_CUDA(ctx, cudaStreamIsCapturing(ctx->stream, &cs));
-    if (!graph || cs != cudaStreamCaptureStatusNone) return lz_enqueue<T>(ctx, b, d);
-    MOED_CUDA(ctx, cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
-    const int rc = lz_enqueue<T>(ctx, b, d);
-    cudaGraph_t g = nullptr;
-    cudaError_t e = cudaStreamEndCapture(ctx->stream, &g);
-    cudaGraphExec_t x = nullptr;
-    if (rc == MO_ED_OK && e == cudaSuccess) e = cudaGraphInstantiate(&x, g, 0);
-    if (g) cudaGraphDestroy(g);
-    if (rc != MO_ED_OK || e != cudaSuccess) {
-        // a capture the runtime refused: the same launches, issued directly
-        cudaGetLastError();
-        if (x) cudaGraphExecDestroy(x);
-        return lz_enqueue<T>(ctx, b, d);
-    }
-    e = cudaGraphLaunch(x, ctx->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-    cudaGraphExecDestroy(x);
-    if (e != cudaSuccess) return cuda_fail(ctx, e, "cudaGraphLaunch");
-    return MO_ED_OK;
-}
-
 int lz_run(mo_ed_ctx *ctx, LzBatch &b, std::vector<std::vector<double>> &a,
            std::vector<std::vector<double>> &bb, std::vector<int> &nstep_calc)
 {
     LzBatchDev d;
     lz_fill_dev(b, d);
     const int nrun = d.nrun;
-    int rc = (b.prec == MO_ED_FP32) ? lz_steps<float>(ctx, b, d, true) : lz_steps<double>(ctx, b, d, true);
+    int rc = (b.prec == MO_ED_FP32) ? lz_steps<float>(ctx, b, d) : lz_steps<double>(ctx, b, d);
     if (rc) return rc;
-    std::vector<double> coef((size_t)2 * (b.nstep + 1) * nrun);
+    std::vector<double> coef((size_t)4 * (b.nstep + 1) * nrun);
     std::vector<int> fl(2 * nrun);
-    MOED_CUDA(ctx, cudaMemcpyAsync(coef.data(), b.coef.p, sizeof(double) * coef.size(),
+    MOED_CUDA(ctx, cudaMemcpyAsync(coef.data(), b.coef, sizeof(double) * coef.size(),
                                    cudaMemcpyDeviceToHost, ctx->stream));
-    MOED_CUDA(ctx, cudaMemcpyAsync(fl.data(), b.flags.p, sizeof(int) * fl.size(),
+    MOED_CUDA(ctx, cudaMemcpyAsync(fl.data(), b.flags, sizeof(int) * fl.size(),
                                    cudaMemcpyDeviceToHost, ctx->stream));
     MOED_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     a.assign(nrun, std::vector<double>(b.nstep + 1, 0.0));
     bb.assign(nrun, std::vector<double>(b.nstep + 1, 0.0));
     nstep_calc.assign(nrun, 0);
     for (int r = 0; r < nrun; ++r) {
-        const double *ar = coef.data() + (size_t)2 * (b.nstep + 1) * r;
+        const double *ar = coef.data() + (size_t)4 * (b.nstep + 1) * r;
         const double *nr = ar + (b.nstep + 1);
         nstep_calc[r] = fl[2 * r + 1];
         for (int j = 0; j <= b.nstep; ++j) {
@@ -393,7 +378,7 @@ int lanczos_reference(mo_ed_ctx *ctx, const Sector &s, const double *h_vec, int 
 }
 
 // The same recurrence inside a caller-provided device region.  Layout, each
-// part starting on a 256-byte boundary: a and nrm [nstep+1] each, the two
+// part starting on a 256-byte boundary: a, nrm, inv, cpl [nstep+1] each, the two
 // flags, the update and H*v partial sums, u_0, u_1 u_2 (adjacent; for FP32
 // runs they first hold the FP64 start vector before its conversion) and w.
 namespace {
@@ -401,17 +386,15 @@ struct LzRegion {
     size_t coef, flags, upd, hv, u0, u12, w, end;
 };
 
-size_t up256(size_t x) { return (x + 255) & ~(size_t)255; }
-
 LzRegion lz_region(const Sector &s, int prec, int nstep, int hv_rows)
 {
     const size_t es = prec == MO_ED_FP32 ? sizeof(float) : sizeof(double);
     const size_t Dp = (size_t)s.Dpad();
-    const size_t upd_n = (Dp + kVecChunk - 1) / kVecChunk;
+    const size_t upd_n = (Dp + vec_chunk((long long)Dp) - 1) / vec_chunk((long long)Dp);
     const size_t hv_n = (size_t)std::max(1, s.dn->nitems.at(hv_rows));
     LzRegion r;
     r.coef = 0;
-    r.flags = up256(r.coef + sizeof(double) * 2 * (size_t)(nstep + 1));
+    r.flags = up256(r.coef + sizeof(double) * 4 * (size_t)(nstep + 1));
     r.upd = up256(r.flags + sizeof(int) * 2);
     r.hv = up256(r.upd + sizeof(double) * upd_n);
     r.u0 = up256(r.hv + sizeof(double) * hv_n);
@@ -476,11 +459,14 @@ int lanczos_reference_in(mo_ed_ctx *ctx, const Sector &s, const double *h_vec, i
     R.w = base + g.w;
     R.D = Dp;
     R.upd_item0 = 0;
-    R.upd_nitems = (int)((Dp + kVecChunk - 1) / kVecChunk);
+    R.chunk = vec_chunk(Dp);
+    R.upd_nitems = (int)((Dp + R.chunk - 1) / R.chunk);
     R.hv_item0 = 0;
     R.hv_nitems = s.dn->nitems.at(lb.hv_rows);
     R.a = (double *)(base + g.coef);
     R.nrm = R.a + (nstep + 1);
+    R.inv = R.nrm + (nstep + 1);
+    R.cpl = R.inv + (nstep + 1);
     R.active = (int *)(base + g.flags);
     R.nstep_calc = R.active + 1;
     R.upd_part = (double *)(base + g.upd);
@@ -493,10 +479,10 @@ int lanczos_reference_in(mo_ed_ctx *ctx, const Sector &s, const double *h_vec, i
         double *stage = (double *)(base + g.u12);
         if (int rc = upload_padded(ctx, s, h_vec, stage, sizeof(double))) return rc;
         if (int rc = convert_f64_to_f32(ctx, stage, (float *)R.u[0], Dp)) return rc;
-        if (int rc = lz_steps<float>(ctx, lb, d, false)) return rc;
+        if (int rc = lz_steps<float>(ctx, lb, d)) return rc;
     } else {
         if (int rc = upload_padded(ctx, s, h_vec, R.u[0], sizeof(double))) return rc;
-        if (int rc = lz_steps<double>(ctx, lb, d, false)) return rc;
+        if (int rc = lz_steps<double>(ctx, lb, d)) return rc;
     }
     MOED_CUDA(ctx, cudaMemcpyAsync(a, R.a, sizeof(double) * (nstep + 1), cudaMemcpyDeviceToHost, ctx->stream));
     MOED_CUDA(ctx, cudaMemcpyAsync(b, R.nrm, sizeof(double) * (nstep + 1), cudaMemcpyDeviceToHost, ctx->stream));

@@ -6,7 +6,10 @@
 namespace moed {
 
 constexpr int kLzMaxRuns = 24;
-constexpr int kVecChunk = 8192;   // elements per item of the elementwise kernels
+// elements per item of the elementwise kernels: enough items to fill the chip
+// first (0.73 million FP64 elements, k_lz_update: 16 us with 8,192 = 90 items,
+// 12 us with 1,024), then few, so that the partials stay few
+inline int vec_chunk(long long n) { return n < (1LL << 22) ? 1024 : 8192; }
 
 // One run of the reference recurrence (ed_lanczos.F90:14-68) on the device.
 // u[0..2] hold u_{j-2}, u_{j-1}, u_j (unnormalized, ring), w = H u_j.
@@ -14,9 +17,11 @@ struct LzRunDev {
     void *u[3];
     void *w;
     long long D;
-    int upd_item0, upd_nitems;    // items of the update kernel (kVecChunk elements)
+    int chunk;                    // elements per item of the update kernel
+    int upd_item0, upd_nitems;    // its items
     int hv_item0, hv_nitems;      // items of the H*v kernel
     double *a, *nrm;              // [nstep+1] device
+    double *inv, *cpl;            // [nstep+1] device: 1 / sqrt(nrm[j]), sqrt(nrm[j] / nrm[j-1])
     int *active;                  // 1 while running
     int *nstep_calc;              // device
     double *upd_part, *hv_part;   // partial sums
@@ -33,10 +38,11 @@ struct LzBatch {
     int prec = MO_ED_FP64;
     int nstep = 0;
     std::vector<Sector> sec;
-    std::vector<DevBuf> vecs;     // 4 per run
-    DevBuf coef;                  // a, nrm per run
-    DevBuf flags;                 // active, nstep_calc per run
-    DevBuf upd_part, hv_part;
+    DevBuf own;                   // workspace of a large batch (small ones use the context's)
+    std::vector<void *> vecs;     // 4 per run
+    double *coef = nullptr;       // a, nrm, inv, cpl per run, nstep + 1 each
+    int *flags = nullptr;         // active, nstep_calc per run
+    double *upd_part = nullptr, *hv_part = nullptr;
     std::vector<int> upd_item0, upd_nitems, hv_item0, hv_nitems;
     int upd_total = 0, hv_total = 0;
     int hv_variant = 0, hv_rows = 0;   // H*v tile shape shared by all runs

@@ -34,6 +34,8 @@
 
 namespace moed {
 
+namespace cg = cooperative_groups;
+
 constexpr int kFitThreads = 128;
 // Frprmn::run's return value for a fit that gave up its cluster to a
 // waiting fit (not an MO_ED code: k_fit parks such fits and resumes them)
@@ -235,22 +237,189 @@ __device__ __forceinline__ double chi2_scale_g(double s, int i, int nx, int norb
     return c * s / (double)(float)(norb * norb) / (double)(float)nw;
 }
 
+// FUNC and dfunc of a batch of parameter sets: a cluster of 1 to 8 CTAs per
+// set, which share its w_n.  Bound by the FP64 pipe (an FP64 warp instruction
+// holds it for 64 cycles), so the sums are arranged for few instructions.
+// With y = 1 / (w^2 + e^2), R = conj-weighted residual r / w_n and
+// u = e Re R + w Im R, from 1/z = -y (e + i w) and y (e^2 + w^2) = 1,
+//   Re[conj(R) / z]   = -y u
+//   Re[conj(R) / z^2] = y (2 e y u - Re R),
+// so a coupling takes 2 instructions forward and 5 backward, V and V^2 come in
+// once per sum, and a level takes 4 in all: 167 per (set, w_n) at 3 x 12 with
+// 12 couplings, where chi2_sums (the fits', whose iterations follow its
+// roundings) takes 240.  A 256-set batch of 512 w_n: 79.9 -> 53 us.
+constexpr int kChiThreads = 128;
+constexpr int kChiSeg = 8;           // segments of a row's final sum
+constexpr int kChiSegLen = kChiThreads / kChiSeg;
+__host__ __device__ inline int chi2_rows(int nbath, int norb) { return 2 * nbath * norb + norb + 1; }
+// Shared memory (doubles, then ints): y [nbath][threads]; the sums' rows
+// [chi2_rows][threads] (|r|^2 / w, so that FUNC is the same with and without
+// dfunc; A = sum y u and B = sum y (2 e y u - Re R) per listed coupling; Re R
+// per orbital); segment sums and sums; x; V^2,
+// V^2 e and 2 e of the listed couplings; their levels and each coupling's place.
+static size_t chi2_batch_smem(int nx, int nbath, int norb)
+{
+    const size_t rows = chi2_rows(nbath, norb), nv = (size_t)nbath * norb;
+    return sizeof(double) * ((nbath + rows) * kChiThreads + rows * (kChiSeg + 1) + nx + 3 * nv) + sizeof(int) * 2 * nv;
+}
+
 // x: [nreq][nx]; dev: Fortran (norb, nw) interleaved complex; f: [nreq];
 // g: [nreq][nx] (written only where want_grad[b] != 0, or all if want_grad null)
-__global__ void __launch_bounds__(kFitThreads, 1)
+__global__ void __launch_bounds__(kChiThreads)
 k_chi2(const double *__restrict__ x, int nx, const int *__restrict__ want_grad, int nw, int norb,
        int nbath, const double *__restrict__ omega, const double *__restrict__ dev, int fcmplx,
-       double *__restrict__ f, double *__restrict__ g)
+       double *__restrict__ f, double *__restrict__ g, int ncta, double scale_f, double scale_g)
 {
-    extern __shared__ double sm[];          // chi2_smem_bytes(nx, nbath, kFitThreads)
-    __shared__ double sums[kMaxX + 1];
-    const int b = blockIdx.x;
+    extern __shared__ double sm[];
+    constexpr int nt = kChiThreads;
+    const int nv = nbath * norb, maxr = chi2_rows(nbath, norb);
+    double *const sy = sm + threadIdx.x;                    // [nbath][nt], this thread's column
+    double *const srow = sm + (size_t)nbath * nt;           // [maxr][nt]
+    double *const red = srow + (size_t)maxr * nt;           // [maxr][kChiSeg]
+    double *const sums = red + maxr * kChiSeg;              // [maxr]
+    double *const sx = sums + maxr;                         // [nx]
+    double *const lv2 = sx + nx, *const lv2e = lv2 + nv, *const le2 = lv2e + nv;   // [nv]
+    int *const lk = (int *)(le2 + nv), *const place = lk + nv;
+    __shared__ int off[kMaxOrb + 1];
+    const int tid = threadIdx.x, b = blockIdx.x / ncta, rank = blockIdx.x - b * ncta;
     const bool grad = g != nullptr && (want_grad ? want_grad[b] != 0 : true);
-    chi2_sums(x + (size_t)b * nx, nx, grad, nw, 0, blockDim.x, norb, nbath, omega, dev, fcmplx, sm, sums);
-    if (threadIdx.x == 0) f[b] = chi2_scale_f(sums[0], norb, nw);
+    for (int i = tid; i < nx; i += nt) sx[i] = x[(size_t)b * nx + i];
+    __syncthreads();
+    const double *eps = sx, *V = sx + nbath, *ef = sx + nx - norb;
+    if (tid < 32) {
+        // warp 0, lane k = bath level k: the couplings that enter orbital a's
+        // sums (chi2_sums), one list for all orbitals
+        const int k = tid;
+        const bool eps_ok = k < nbath && finite_bits(eps[k]);
+        int c = 0;
+        for (int a = 0; a < norb; ++a) {
+            const double v = k < nbath ? V[a * nbath + k] : 0.0;
+            const bool keep = k < nbath && ((__double_as_longlong(v) << 1) != 0 || !eps_ok);
+            const unsigned m = __ballot_sync(0xffffffffu, keep);
+            if (k == 0) off[a] = c;
+            if (k < nbath) place[a * nbath + k] = keep ? c + __popc(m & ((1u << k) - 1u)) : -1;
+            if (keep) {
+                const int s = c + __popc(m & ((1u << k) - 1u));
+                lk[s] = k;
+                // V^2 e to the last bit, as its error would enter every w_n alike
+                const double v2 = v * v, p = v2 * eps[k];
+                const double r = fma(fma(v, v, -v2), eps[k], fma(v2, eps[k], -p));
+                lv2[s] = v2;
+                lv2e[s] = finite_bits(r) ? p + r : p;
+                le2[s] = eps[k] + eps[k];
+            }
+            c += __popc(m);
+        }
+        if (k == 0) off[norb] = c;
+    }
+    __syncthreads();
+    const int nc = off[norb];
+    double *const sA = srow + nt + tid, *const sB = sA + (size_t)nc * nt;   // this thread's columns
     if (grad)
-        for (int i = threadIdx.x; i < nx; i += blockDim.x)
-            g[(size_t)b * nx + i] = chi2_scale_g(sums[1 + i], i, nx, norb, nbath, nw);
+        for (int i = 0; i < 2 * nc; ++i) sA[(size_t)i * nt] = 0.0;
+    double fsum = 0.0, gef[kMaxOrb];
+#pragma unroll
+    for (int a = 0; a < kMaxOrb; ++a) gef[a] = 0.0;
+    for (int n = rank * nt + tid; n < nw; n += ncta * nt) {
+        const double w = omega[n];
+        double Dr[kMaxOrb], Di[kMaxOrb];
+#pragma unroll
+        for (int a = 0; a < kMaxOrb; ++a)
+            if (a < norb) {
+                Dr[a] = dev[2 * ((size_t)n * norb + a)];
+                Di[a] = dev[2 * ((size_t)n * norb + a) + 1];
+            }
+        const double wz = fcmplx ? widen((float)w) : w;
+        const double wz2 = wz * wz;
+        const double inv_w = rcp_pos(w);
+#pragma unroll 4
+        for (int k = 0; k < nbath; ++k) sy[k * nt] = rcp_pos(fma(eps[k], eps[k], wz2));
+#pragma unroll
+        for (int a = 0; a < kMaxOrb; ++a) {
+            if (a < norb) {
+                const int s0 = off[a], s1 = off[a + 1];
+                double S0 = 0.0, S1 = 0.0;
+#pragma unroll 4
+                for (int s = s0; s < s1; ++s) {
+                    const double y = sy[lk[s] * nt];
+                    S0 = fma(lv2[s], y, S0);
+                    S1 = fma(lv2e[s], y, S1);
+                }
+                const double rr = (ef[a] - S1) - Dr[a], ri = fma(-wz, S0, -Di[a]);
+                const double Rr = rr * inv_w, Ri = ri * inv_w;
+                fsum = fma(rr, Rr, fma(ri, Ri, fsum));
+                if (grad) {
+                    const double wRi = wz * Ri;
+                    gef[a] += Rr;
+#pragma unroll 4
+                    for (int s = s0; s < s1; ++s) {
+                        const double e = eps[lk[s]], y = sy[lk[s] * nt];
+                        const double yu = y * fma(e, Rr, wRi);
+                        sA[s * nt] += yu;
+                        sB[s * nt] = fma(y, fma(le2[s], yu, -Rr), sB[s * nt]);
+                    }
+                }
+            }
+        }
+    }
+    // rows in fixed segments, then the segments, then the CTAs
+    const int nr = grad ? 1 + 2 * nc + norb : 1;
+    if (grad) {
+#pragma unroll
+        for (int a = 0; a < kMaxOrb; ++a)
+            if (a < norb) sA[(size_t)(2 * nc + a) * nt] = gef[a];
+    }
+    srow[tid] = fsum;
+    __syncthreads();
+    for (int i = tid; i < nr * kChiSeg; i += nt) {
+        const double *c = srow + (size_t)i * kChiSegLen;
+        double s[kChiSegLen];
+#pragma unroll
+        for (int t = 0; t < kChiSegLen; ++t) s[t] = c[(t + i) & (kChiSegLen - 1)];   // rotated: no bank conflicts
+#pragma unroll
+        for (int h = kChiSegLen / 2; h; h >>= 1)
+#pragma unroll
+            for (int t = 0; t < h; ++t) s[t] += s[t + h];
+        red[i] = s[0];
+    }
+    __syncthreads();
+    for (int r = tid; r < nr; r += nt) {
+        const double *q = red + r * kChiSeg;
+        sums[r] = ((q[0] + q[1]) + (q[2] + q[3])) + ((q[4] + q[5]) + (q[6] + q[7]));
+    }
+    if (ncta == 1) {
+        __syncthreads();
+    } else {
+        cg::cluster_group cl = cg::this_cluster();
+        cl.sync();
+        if (rank == 0)
+            for (int r = tid; r < nr; r += nt) {
+                double s = 0.0;
+                for (int q = 0; q < ncta; ++q) s += cl.map_shared_rank(sums, q)[r];
+                red[r] = s;
+            }
+        cl.sync();
+        if (rank) return;
+    }
+    const double *tot = ncta == 1 ? sums : red;
+    if (tid == 0) f[b] = tot[0] / scale_f;
+    if (grad)
+        for (int i = tid; i < nx; i += nt) {
+            double s = 0.0, c = scale_g;   // 2 / norb^2 / nw (func.f90:128-140)
+            if (i < nbath) {
+                for (int a = 0; a < norb; ++a) {
+                    const int q = place[a * nbath + i];
+                    if (q >= 0) s = fma(lv2[q], tot[1 + nc + q], s);
+                }
+            } else if (i < nx - norb) {
+                const int q = place[i - nbath];
+                if (q >= 0) s = -(sx[i] * tot[1 + q]);
+                c = scale_g + scale_g;
+            } else {
+                s = tot[1 + 2 * nc + i - (nx - norb)];
+            }
+            g[(size_t)b * nx + i] = c * s;
+        }
 }
 
 // calc_dev (ed_green.F90:260-273)
@@ -280,18 +449,47 @@ static int chi2_smem(mo_ed_ctx *ctx, const void *kernel, int nx, int nbath, int 
     return MO_ED_OK;
 }
 
+// k_chi2 over nbatch sets.  A set is split over 2, 4, 8 CTAs while threads
+// have more than one w_n and, for 4 and 8, every CTA finds an SM of its own
+// (larger clusters two to an SM leave a part wave).  3 x 12, 512 w_n, 1 / 2 /
+// 4 / 8 CTAs: 1 set 41 / 26 / 17 / 17 us, 38 sets 41 / 27 / 23 / 31, 152 sets
+// 42 / 35 / 55 / 86, 256 sets 58 / 66 / 76 / 135.
+static int chi2_launch(mo_ed_ctx *ctx, int nbatch, const double *x, int nx, const int *want, int nw, int norb,
+                       int nbath, const double *omega, const double *dev, double *f, double *g)
+{
+    if (nbath < 0) return fail(ctx, MO_ED_ERR_ARG, "bad arguments");
+    const size_t smem = chi2_batch_smem(nx, nbath, norb);
+    MOED_CUDA(ctx, cudaFuncSetAttribute((const void *)k_chi2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    int ncta = 1;
+    while (ncta < 8 && nw > ncta * kChiThreads &&
+           2LL * nbatch * ncta <= (ncta == 1 ? 2 : 1) * ctx->num_sms)
+        ncta *= 2;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)ncta;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)nbatch * ncta);
+    cfg.blockDim = dim3(kChiThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = ctx->stream;
+    cfg.attrs = attr;
+    cfg.numAttrs = ncta > 1 ? 1 : 0;
+    MOED_CUDA(ctx, cudaLaunchKernelEx(&cfg, k_chi2, x, nx, want, nw, norb, nbath, omega, dev,
+                                      ctx->opt.fortran_cmplx, f, g, ncta, (double)(float)(norb * norb * nw),
+                                      2.0 / (double)(float)(norb * norb) / (double)(float)nw));
+    MOED_CHECK_LAUNCH(ctx);
+    return MO_ED_OK;
+}
+
 int chi2_grad_dev(mo_ed_ctx *ctx, int nbatch, const double *x, int nwloc, int ns, int nxsize,
                   const double *omega, const double *dev, int nbath, int norb, double *f, double *g,
                   int want_grad)
 {
     (void)ns;
     if (nbatch <= 0) return MO_ED_OK;
-    size_t smem;
-    if (int rc = chi2_smem(ctx, (const void *)k_chi2, nxsize, nbath, kFitThreads, &smem)) return rc;
-    k_chi2<<<nbatch, kFitThreads, smem, ctx->stream>>>(x, nxsize, nullptr, nwloc, norb, nbath, omega, dev,
-                                                       ctx->opt.fortran_cmplx, f, want_grad ? g : nullptr);
-    MOED_CHECK_LAUNCH(ctx);
-    return MO_ED_OK;
+    return chi2_launch(ctx, nbatch, x, nxsize, nullptr, nwloc, norb, nbath, omega, dev, f, want_grad ? g : nullptr);
 }
 
 // ---------------------------------------------------------------------------
@@ -339,13 +537,10 @@ struct Evaluator {
         }
         MOED_CUDA(ctx, cudaMemcpyAsync(dx.p, x, sizeof(double) * nreq * nx, cudaMemcpyHostToDevice, ctx->stream));
         MOED_CUDA(ctx, cudaMemcpyAsync(dw.p, want, sizeof(int) * nreq, cudaMemcpyHostToDevice, ctx->stream));
-        size_t smem;
-        if (int rc = chi2_smem(ctx, (const void *)k_chi2, nx, P->nbath, kFitThreads, &smem)) return rc;
-        k_chi2<<<nreq, kFitThreads, smem, ctx->stream>>>((const double *)dx.p, nx, (const int *)dw.p, P->nwloc,
-                                                         P->norb, P->nbath, (const double *)P->omega.p,
-                                                         (const double *)P->dev.p, ctx->opt.fortran_cmplx,
-                                                         (double *)df.p, (double *)dg.p);
-        MOED_CHECK_LAUNCH(ctx);
+        if (int rc = chi2_launch(ctx, nreq, (const double *)dx.p, nx, (const int *)dw.p, P->nwloc, P->norb, P->nbath,
+                                 (const double *)P->omega.p, (const double *)P->dev.p, (double *)df.p,
+                                 (double *)dg.p))
+            return rc;
         MOED_CUDA(ctx, cudaMemcpyAsync(f, df.p, sizeof(double) * nreq, cudaMemcpyDeviceToHost, ctx->stream));
         if (g)
             MOED_CUDA(ctx, cudaMemcpyAsync(g, dg.p, sizeof(double) * nreq * nx, cudaMemcpyDeviceToHost, ctx->stream));
@@ -580,7 +775,6 @@ constexpr int kFitCta = 256;
 constexpr int kFitMaxCluster = 8;
 constexpr size_t kFitSmemMax = 220 * 1024;
 
-namespace cg = cooperative_groups;
 
 // Scheduler words of one k_fit launch (global memory, zeroed before it):
 // q[kQFresh] fits handed out from the batch, q[kQParked] fits parked,

@@ -33,11 +33,16 @@
 #include <cmath>
 #include <cstring>
 
+#include <cooperative_groups.h>
+
+#include "hvrow.cuh"
 #include "math64.cuh"
 #include "symeig.h"
 #include "vecops.cuh"
 
 namespace moed {
+
+namespace cg = cooperative_groups;
 
 constexpr int kKryMax = 352;                           // Krylov vectors of one run
 constexpr size_t kKryRunBytes = (size_t)48 << 30;      // and their memory (at most half of what is free)
@@ -45,6 +50,12 @@ constexpr long long kKryMinDim = 128;                  // smaller sectors: thick
 constexpr size_t kKryPoolBytes = (size_t)4 << 30;      // Krylov vectors kept in the context between solves
 constexpr size_t kRrPoolBytes = (size_t)64 << 20;      // largest FP64 vector of the pooled Rayleigh-Ritz workspace
 constexpr size_t kSlabBytes = (size_t)1 << 20;         // returned vectors up to this size share one allocation
+// k_kry_cluster: sectors up to these sizes, shared memory of a CTA.  4 states
+// by launches / by clusters, ms: FP32 4,900 elements 2.5 / 1.5, 10,584 4.3 / 3.3,
+// 15,876 3.1 / 2.7; FP64 4,900 3.8 / 3.0, 7,056 4.9 / 4.4, 10,584 6.2 / 6.9
+// (8 SMs' FP64 pipes are the limit there).
+constexpr long long kKcMaxDimF32 = 16384, kKcMaxDimF64 = 8192;
+constexpr int kKcSmem = 80 * 1024;
 // partial sums that the next step's blocks add themselves; with more, a
 // one-block launch does
 constexpr int kKryFuseParts = 1536;
@@ -148,6 +159,174 @@ k_kry_update(KryScal sc, int j, const double *__restrict__ norm_part, int gn, co
     acc += (double)sacc;
     const double t = block_sum(acc, sred);
     if (threadIdx.x == 0) norm_out[blockIdx.x] = t;
+}
+
+// ---------------------------------------------------------------------------
+// small sectors: many steps in one launch
+// ---------------------------------------------------------------------------
+// Steps j0 .. j1 of a run by one cluster; U[i] is U_{j0-2+i}.
+struct KrySeg {
+    static constexpr int most = 32;      // steps
+    int j0, j1;
+    bool update0, hv1;                   // U_{j0} is to be formed; w = H U_{j1} as well
+    const double *norm_part;             // !update0: partials of ||U_{j0}||^2
+    int gn;
+    void *U[most + 2];
+    void *w;
+};
+
+// The recurrence of k_kry_update and k_hv_row for sectors that a cluster of up
+// to 8 CTAs holds: a launch per 2 x steps becomes one per segment between
+// reorthogonalisations.  A thread keeps its EPT elements of w, U_{j-1}, U_{j-2}
+// in registers; U_j goes to every CTA's shared memory, so the gathers of H*v
+// are local; two cluster barriers per step.  What bounds a step is its chain of
+// latencies (barriers, two FP64 sums, the scalars), not work: 4,900 FP32
+// elements, 10 us per step as two launches, 4.8 us so.
+constexpr int kKcThreads = 512, kKcMaxEpt = 4;
+template <typename T, int EPT>
+__global__ void __launch_bounds__(kKcThreads)
+k_kry_cluster(const __grid_constant__ HvJobT<T> jb, const ModelDev *__restrict__ mdl, KryScal sc,
+              const __grid_constant__ KrySeg seg, int ld)
+{
+    constexpr int NT = kKcThreads;
+    extern __shared__ double raw[];
+    double *const red = raw;                               // [2][NT]
+    T *const xs = (T *)(red + 2 * NT);                     // U_j without its pads (jb.ld = nu)
+    __shared__ T s_cross[kMaxImp * kMaxImp];
+    __shared__ unsigned s_pmask[kMaxImp];
+    __shared__ int s_t4[kMaxPair * kMaxImp];
+    __shared__ double s_slot[2 * 8], s_part[4], s_n0;
+    __shared__ T s_coef[3];
+    cg::cluster_group cl = cg::this_cluster();
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, C = gridDim.x, rank = blockIdx.x;
+    const int nimp = mdl->nimp, npair = mdl->npair, nu = jb.nu, n = nu * jb.nd;
+    for (int i = tid; i < npair * nimp; i += NT) s_t4[i] = mdl->t4[i];
+    for (int i = tid; i < nimp; i += NT) s_pmask[i] = mdl->pairmask[i];
+    for (int i = tid; i < nimp * nimp; i += NT) s_cross[i] = (T)mdl->cross[i];
+    const T Jc = (T)mdl->J;
+    if (!seg.update0 && wid == 0) {
+        double a = 0.0;
+        for (int i = lane; i < seg.gn; i += 32) a += seg.norm_part[i];
+        a = warp_sum(a);
+        if (lane == 0) s_n0 = a;
+    }
+    __syncthreads();
+    // this thread's elements: address, column and row information, diagonal
+    int at[EPT], col[EPT], row[EPT], inf[EPT], dinf[EPT];
+    T diag[EPT], w[EPT], uc[EPT], up[EPT];
+    const T *gw = (const T *)seg.w, *g1 = (const T *)seg.U[1], *g2 = (const T *)seg.U[0], *g0 = (const T *)seg.U[2];
+#pragma unroll
+    for (int k = 0; k < EPT; ++k) {
+        const int e = (k * C + rank) * NT + tid;
+        at[k] = -1;
+        w[k] = uc[k] = up[k] = T(0);
+        if (e < n) {
+            const int d = e / nu, u = e - d * nu;
+            at[k] = d * ld + u;
+            row[k] = d;
+            col[k] = u;
+            inf[k] = __ldg(jb.up_info + u);
+            dinf[k] = __ldg(jb.dn_info + d);
+            diag[k] = __ldg(jb.up_diag + u) + __ldg(jb.dn_diag + d) +
+                      s_cross[((inf[k] >> 8) & 0xff) * nimp + ((dinf[k] >> 8) & 0xff)];
+            if (seg.update0) {
+                w[k] = gw[at[k]];
+                uc[k] = g1[at[k]];
+                if (seg.j0 >= 2) up[k] = g2[at[k]];
+            } else {
+                uc[k] = g0[at[k]];
+                if (seg.j0 >= 1) up[k] = g1[at[k]];
+            }
+        }
+    }
+    double inv1 = 0.0;   // thread 0: inv of the step before the one to come
+    if (tid == 0) {
+        const int j = seg.j0 - 1;
+        if (j >= 0) inv1 = sc.inv[j];
+        if (seg.update0) {
+            s_coef[0] = (T)inv1;
+            s_coef[1] = (T)sc.alpha[j];
+            s_coef[2] = j >= 1 ? (T)(sc.beta[j] * sc.inv[j - 1]) : T(0);
+        }
+    }
+    cl.sync();           // every CTA runs; the coefficients are there
+    for (int j = seg.j0;; ++j) {
+        const bool given = j == seg.j0 && !seg.update0;
+        T sq = T(0);
+        if (!given) {
+            const T s = s_coef[0], a = s_coef[1], c = s_coef[2];
+            T *un = (T *)seg.U[j - seg.j0 + 2];
+#pragma unroll
+            for (int k = 0; k < EPT; ++k)
+                if (at[k] >= 0) {
+                    const T v = s * (w[k] - a * uc[k]) - c * up[k];
+                    up[k] = uc[k];
+                    uc[k] = v;
+                    sq += v * v;
+                    un[at[k]] = v;
+                }
+            for (int d = rank * (NT / 32) + wid; d < jb.nd; d += C * (NT / 32))
+                for (int u = nu + lane; u < ld; u += 32) un[d * ld + u] = T(0);
+        }
+        if (j == seg.j1 && !seg.hv1) break;
+        for (int r = 0; r < C; ++r) {
+            T *peer = cl.map_shared_rank(xs, r);
+#pragma unroll
+            for (int k = 0; k < EPT; ++k)
+                if (at[k] >= 0) peer[(k * C + rank) * NT + tid] = uc[k];
+        }
+        cl.sync();
+        double dot = 0.0;
+#pragma unroll
+        for (int k = 0; k < EPT; ++k)
+            if (at[k] >= 0) {
+                w[k] = hv_moves<T, T, false>(jb, mdl, xs, row[k], col[k], inf[k], dinf[k], s_pmask, s_t4, nimp, Jc,
+                                             diag[k] * uc[k]);
+                const double p = widen(uc[k] * w[k]);
+                dot = k == 0 ? p : dot + p;
+            }
+        // sums over the cluster in a fixed order: halves of each by a warp
+        red[tid] = widen(sq);
+        red[NT + tid] = dot;
+        __syncthreads();
+        if (wid < 4) {
+            const double *p = red + wid * (NT / 2) + lane;
+            double v = 0.0;
+#pragma unroll
+            for (int i = 0; i < NT / 2; i += 32) v += p[i];
+            v = warp_sum(v);
+            if (lane == 0) s_part[wid] = v;
+        }
+        __syncthreads();
+        if (tid < 2 * C) cl.map_shared_rank(s_slot, tid >> 1)[2 * rank + (tid & 1)] = s_part[2 * (tid & 1)] + s_part[2 * (tid & 1) + 1];
+        cl.sync();
+        if (wid == 0) {
+            double v = lane < 2 * C ? s_slot[lane] : 0.0;
+#pragma unroll
+            for (int o = 8; o > 1; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+            const double d = __shfl_sync(0xffffffffu, v, 1), n2 = given ? s_n0 : v;
+            if (lane == 0) {
+                const double in = rsqrt_pos(n2), be = n2 * in, al = d * rcp_pos(n2);
+                if (rank == 0) {
+                    sc.alpha[j] = al;
+                    sc.beta[j] = be;
+                    sc.inv[j] = in;
+                }
+                s_coef[0] = (T)in;
+                s_coef[1] = (T)al;
+                s_coef[2] = j >= 1 ? (T)(be * inv1) : T(0);
+                inv1 = in;
+            }
+        }
+        __syncthreads();
+        if (j == seg.j1) {
+            T *gwo = (T *)seg.w;
+#pragma unroll
+            for (int k = 0; k < EPT; ++k)
+                if (at[k] >= 0) gwo[at[k]] = w[k];
+            break;
+        }
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -428,6 +607,9 @@ struct KryRun {
     size_t vb;
     int kind, G, Gr, gmax, gd = 0;
     bool fused = false;
+    bool clustered = false;       // segments of steps by k_kry_cluster
+    int csize = 1, ept = 1;
+    HvJobT<T> job;
     KryVectors U;
     DevBuf wlocal;
     T *w = nullptr;
@@ -470,6 +652,15 @@ struct KryRun {
     {
         if (int rc = hv_dot_parts(ctx, s, kind, &gd)) return rc;
         fused = gmax + gd <= kKryFuseParts;
+        if (s.D() <= (f32 ? kKcMaxDimF32 : kKcMaxDimF64)) {
+            if (int rc = hv_row_job<T>(ctx, s, kind, &job, &clustered)) return rc;
+            job.ld = job.nu;
+            while (csize < 8 && s.D() > (long long)csize * kKcThreads) csize *= 2;
+            ept = (int)((s.D() + (long long)csize * kKcThreads - 1) / ((long long)csize * kKcThreads));
+            const void *k = ept == 1 ? (const void *)k_kry_cluster<T, 1>
+                                     : ept == 2 ? (const void *)k_kry_cluster<T, 2> : (const void *)k_kry_cluster<T, kKcMaxEpt>;
+            MOED_CUDA(ctx, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kKcSmem));
+        }
         std::vector<DevBuf> &sm = ctx->kry_small;
         if (sm.size() < 4) sm.resize(4);
         // scalars, two sets of norm partials, dot partials; multi-dot partials and sums; h columns; w
@@ -521,21 +712,41 @@ struct KryRun {
         return axpys<T, NW>(ctx, P, nf + n, src, rows, sc.inv - nf, x, Dp, norm_out, h, ns);
     }
 
+    // U_0: a random vector, orthogonal to the front vectors
+    int first()
+    {
+        if (int rc = U.grow(1)) return rc;
+        T *un = (T *)U.p[0];
+        k_random<T><<<Gr, kVecThreads, 0, ctx->stream>>>(un, Dp, s.ld(), s.up->n, seed);
+        MOED_CHECK_LAUNCH(ctx);
+        if (front.empty()) {
+            gn = Gr;
+            k_dot_part<T, T><<<Gr, kVecThreads, 0, ctx->stream>>>(un, un, Dp, npart[0]);
+            MOED_CHECK_LAUNCH(ctx);
+        } else {
+            for (int pass = 0; pass < 2; ++pass)
+                if (int rc = clean<1>(0, WPtrs<T>{{un, nullptr}}, npart[0], hcol)) return rc;
+        }
+        return MO_ED_OK;
+    }
+
+    // U_{j-1} and U_j together: one pass over the others for both
+    int reorthogonalise(int j)
+    {
+        if (int rc = clean<2>(j - 1, WPtrs<T>{{(T *)U.p[j - 1], (T *)U.p[j]}}, npart[j & 1], hcol + (size_t)(j - 1) * ns))
+            return rc;
+        re.push_back({j, j - std::max(last_re, base)});
+        last_re = j;
+        next_re = j + period;
+        return MO_ED_OK;
+    }
+
     int step(int j)
     {
         if (int rc = U.grow(j + 1)) return rc;
         T *un = (T *)U.p[j];
         if (j == 0) {
-            k_random<T><<<Gr, kVecThreads, 0, ctx->stream>>>(un, Dp, s.ld(), s.up->n, seed);
-            MOED_CHECK_LAUNCH(ctx);
-            if (front.empty()) {
-                gn = Gr;
-                k_dot_part<T, T><<<Gr, kVecThreads, 0, ctx->stream>>>(un, un, Dp, npart[0]);
-                MOED_CHECK_LAUNCH(ctx);
-            } else {
-                for (int pass = 0; pass < 2; ++pass)
-                    if (int rc = clean<1>(0, WPtrs<T>{{un, nullptr}}, npart[0], hcol)) return rc;
-            }
+            if (int rc = first()) return rc;
         } else {
             T *uc = (T *)U.p[j - 1];
             const T *up = j >= 2 ? (const T *)U.p[j - 2] : nullptr;
@@ -548,19 +759,77 @@ struct KryRun {
                                                                            npart[j & 1]);
             MOED_CHECK_LAUNCH(ctx);
             gn = G;
-            if (j >= next_re) {
-                // U_{j-1} and U_j together: one pass over the others for both
-                if (int rc = clean<2>(j - 1, WPtrs<T>{{uc, un}}, npart[j & 1], hcol + (size_t)(j - 1) * ns)) return rc;
-                re.push_back({j, j - std::max(last_re, base)});
-                last_re = j;
-                next_re = j + period;
-            }
+            if (j >= next_re)
+                if (int rc = reorthogonalise(j)) return rc;
         }
         if (int rc = hv_single_dot(ctx, s, kind, un, w, dpart)) return rc;
         ++matvecs;
         if (!fused) {
             k_kry_scalars<<<1, kVecThreads, 0, ctx->stream>>>(sc, j, npart[j & 1], gn, dpart, gd);
             MOED_CHECK_LAUNCH(ctx);
+        }
+        redo = -1;
+        return MO_ED_OK;
+    }
+
+    size_t kc_smem() const { return sizeof(double) * 2 * kKcThreads + sizeof(T) * (size_t)s.D(); }
+
+    template <int EPT>
+    int segment(const KrySeg &seg)
+    {
+        const size_t smem = kc_smem();
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = (unsigned)csize;
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = 1;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)csize);
+        cfg.blockDim = dim3(kKcThreads);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = ctx->stream;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        MOED_CUDA(ctx, cudaLaunchKernelEx(&cfg, k_kry_cluster<T, EPT>, job, (const ModelDev *)ctx->d_mdl, sc, seg, s.ld()));
+        MOED_CHECK_LAUNCH(ctx);
+        return MO_ED_OK;
+    }
+
+    // steps j .. stop - 1 in segments: up to the next vector to be
+    // reorthogonalised, and on from its H*v
+    int run_to(int &j, int stop)
+    {
+        bool formed = false;             // U_j is there and its H*v is not
+        while (j < stop) {
+            if (j == 0 && !formed) {
+                if (int rc = first()) return rc;
+                formed = true;
+            }
+            KrySeg seg;
+            memset(&seg, 0, sizeof(seg));
+            const bool clean_last = !formed ? std::max(j, next_re) < std::min(stop, j + KrySeg::most)
+                                            : std::max(j + 1, next_re) < std::min(stop, j + KrySeg::most);
+            const int last = clean_last ? std::max(formed ? j + 1 : j, next_re) : std::min(stop, j + KrySeg::most) - 1;
+            if (int rc = U.grow(last + 1)) return rc;
+            seg.j0 = j;
+            seg.j1 = last;
+            seg.update0 = !formed;
+            seg.hv1 = !clean_last;
+            seg.norm_part = npart[j & 1];
+            seg.gn = gn;
+            for (int i = 0; i < last - j + 3; ++i)
+                if (j - 2 + i >= 0) seg.U[i] = U.p[j - 2 + i];
+            seg.w = w;
+            if (int rc = ept == 1 ? segment<1>(seg) : ept == 2 ? segment<2>(seg) : segment<kKcMaxEpt>(seg)) return rc;
+            matvecs += last - j + (clean_last ? 0 : 1);
+            if (clean_last) {
+                if (int rc = reorthogonalise(last)) return rc;
+                j = last;
+                formed = true;
+            } else {
+                j = last + 1;
+                formed = false;
+            }
         }
         redo = -1;
         return MO_ED_OK;
@@ -583,7 +852,7 @@ struct KryRun {
     int read_j[2], read_re[2], read_gap[2];
     int read_back(int slot, int j)
     {
-        if (fused) {
+        if (fused && !clustered) {
             k_kry_scalars<<<1, kVecThreads, 0, ctx->stream>>>(sc, j, npart[j & 1], gn, dpart, gd);
             MOED_CHECK_LAUNCH(ctx);
         }
@@ -628,6 +897,8 @@ struct KryRun {
         int nread = 0, ndone = 0;     // reads issued, reads judged
         for (;;) {
             if (!full) {
+                if (clustered)
+                    if (int rc = run_to(j, stop)) return rc == MO_ED_ERR_NOMEM ? (int)MO_ED_OK : rc;
                 for (; j < stop; ++j)
                     if (int rc = step(j)) {
                         if (rc != MO_ED_ERR_NOMEM || j < least + 8) return rc == MO_ED_ERR_NOMEM ? (int)MO_ED_OK : rc;

@@ -47,6 +47,7 @@
 #include <mutex>
 #include <tuple>
 
+#include "hvrow.cuh"
 #include "internal.h"
 #include "math64.cuh"
 
@@ -1254,62 +1255,17 @@ k_hv_row(const __grid_constant__ HvBatch<TA> batch, const ModelDev *__restrict__
         const TX *__restrict__ x = (const TX *)jb.x;
         const TX *__restrict__ xd = x + (size_t)d * ld;
         TY *__restrict__ y = (TY *)jb.y + (size_t)d * ld;
-        const int dinf = __ldg(jb.dn_info + d), id = (dinf >> 8) & 0xff, dcnt = dinf & 0xff;
+        const int dinf = __ldg(jb.dn_info + d), id = (dinf >> 8) & 0xff;
         const TA ddiag = __ldg(jb.dn_diag + d);
         __syncthreads();   // the previous row is done with s_cross and s_red
         for (int i = tid; i < nimp; i += NT) s_cross[i] = (TA)mdl->cross[i * nimp + id];
         __syncthreads();
         double dacc = 0.0;
         for (int u = tid; u < ld; u += NT) {
-            const int inf = __ldg(jb.up_info + u), iu = (inf >> 8) & 0xff, cnt = inf & 0xff;
+            const int inf = __ldg(jb.up_info + u), iu = (inf >> 8) & 0xff;
             const TX xv = __ldg(xd + u);
-            TA acc = (__ldg(jb.up_diag + u) + ddiag + s_cross[iu]) * (TA)xv;
-            // up-spin moves of the column, 4 at a time
-            const HopEnt<TA> *tab = jb.up_tab + (size_t)(u >> 2) * jb.up_hw * 4 + (u & 3);
-            for (int s0 = 0; s0 < cnt; s0 += 4) {
-                HopEnt<TA> e[4];
-                TX g[4];
-#pragma unroll
-                for (int t = 0; t < 4; ++t) e[t] = tab[4 * min(s0 + t, cnt - 1)];
-#pragma unroll
-                for (int t = 0; t < 4; ++t) g[t] = __ldg(xd + e[t].t);
-#pragma unroll
-                for (int t = 0; t < 4; ++t)
-                    if (s0 + t < cnt) acc += e[t].v * (TA)g[t];
-            }
-            // down-spin moves of the row
-            for (int s0 = 0; s0 < dcnt; s0 += 4) {
-                TA v[4];
-                TX g[4];
-#pragma unroll
-                for (int t = 0; t < 4; ++t) {
-                    const int s = min(s0 + t, dcnt - 1);
-                    v[t] = __ldg(jb.dn_val + (size_t)s * jb.nd + d);
-                    g[t] = __ldg(x + (size_t)__ldg(jb.dn_tgt + (size_t)s * jb.nd + d) * ld + u);
-                }
-#pragma unroll
-                for (int t = 0; t < 4; ++t)
-                    if (s0 + t < dcnt) acc += v[t] * (TA)g[t];
-            }
-            // spin-flip and pair hopping
-            unsigned pm = s_pmask[iu];
-            while (pm) {
-                const int p = __ffs(pm) - 1;
-                pm &= pm - 1;
-                const int e = s_t4[p * nimp + iu];
-                const TX *xu = x + u + (int)(short)(e & 0xffff);
-                const TA c = (e & 0x40000000) ? -Jc : Jc;
-                const int esf = s_t4[mdl->pair_rev[p] * nimp + id];   // spin-flip: T_{j<-i}(d)
-                const int eph = s_t4[p * nimp + id];                  // pair hop:  T_{i<-j}(d)
-                if (esf < 0) {
-                    const TX g = __ldg(xu + (size_t)(d + (int)(short)(esf & 0xffff)) * ld);
-                    acc += ((esf & 0x40000000) ? -c : c) * (TA)g;
-                }
-                if (eph < 0) {
-                    const TX g = __ldg(xu + (size_t)(d + (int)(short)(eph & 0xffff)) * ld);
-                    acc += ((eph & 0x40000000) ? -c : c) * (TA)g;
-                }
-            }
+            const TA acc = hv_moves<TX, TA, true>(jb, mdl, x, d, u, inf, dinf, s_pmask, s_t4, nimp, Jc,
+                                                  (__ldg(jb.up_diag + u) + ddiag + s_cross[iu]) * (TA)xv);
             y[u] = (TY)acc;
             if (jb.dot_partial) dacc += (double)((TA)xv * (TA)(TY)acc);
         }
@@ -2422,6 +2378,20 @@ int hv_dot_parts(mo_ed_ctx *ctx, const Sector &s, int kind, int *nparts)
     *nparts = s.dn->nitems.at(R);
     return MO_ED_OK;
 }
+
+// The tables of a sector whose H*v is k_hv_row (*row), for kernels that apply
+// H to their own vectors.
+template <typename TA>
+int hv_row_job(mo_ed_ctx *ctx, const Sector &s, int kind, HvJobT<TA> *job, bool *row)
+{
+    int v;
+    if (int rc = hv_prepare(ctx, s, kind, &v, nullptr)) return rc;
+    *row = v == (kind == HV_F32 ? kRowVarF32 : kRowVarF64);
+    if (*row) hv_fill_job<TA>(ctx, s, variant(kind, v).key(), nullptr, nullptr, *job);
+    return MO_ED_OK;
+}
+template int hv_row_job<float>(mo_ed_ctx *, const Sector &, int, HvJobT<float> *, bool *);
+template int hv_row_job<double>(mo_ed_ctx *, const Sector &, int, HvJobT<double> *, bool *);
 
 int hv_single_dot(mo_ed_ctx *ctx, const Sector &s, int kind, const void *x, void *y, double *dot)
 {

@@ -395,6 +395,8 @@ int hv_single(mo_ed_ctx *ctx, const Sector &s, int kind, const void *x, void *y)
 int hv_multi(mo_ed_ctx *ctx, const Sector &s, int kind, int n, const void *const *x, void *const *y);
 // y = H x with the partials of x . y in dot[0 .. hv_dot_parts); kind HV_F32 or HV_F64.
 int hv_dot_parts(mo_ed_ctx *ctx, const Sector &s, int kind, int *nparts);
+template <typename TA>
+int hv_row_job(mo_ed_ctx *ctx, const Sector &s, int kind, HvJobT<TA> *job, bool *row);
 int hv_single_dot(mo_ed_ctx *ctx, const Sector &s, int kind, const void *x, void *y, double *dot);
 
 // ---- Krylov (krylov.cu) -----------------------------------------------------

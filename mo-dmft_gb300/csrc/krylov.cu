@@ -19,7 +19,9 @@
 #include <cmath>
 #include <cstring>
 
+#include "hvrow.cuh"
 #include "krylov.cuh"
+#include "math64.cuh"
 #include "symeig.h"
 #include "vecops.cuh"
 
@@ -556,6 +558,103 @@ static int orthogonalize(mo_ed_ctx *ctx, const std::vector<DevBuf *> &basis, int
     return MO_ED_OK;
 }
 
+// Steps k .. ncv - 1 of a cycle (H*v, two Gram-Schmidt passes against V_0 ..
+// V_j, column j of the projected matrix, V_{j+1}) in one CTA, for sectors of
+// up to kTsMaxDim elements: seven launches per step otherwise, 25 us of
+// latency.  V_j and w are in shared memory (without row
+// pads: jb.ld = nu), the earlier vectors in L1; a warp per dot.  start: w of
+// the first vector, normalised here (else V_k is given).  A step of 70
+// elements: 6 us.
+constexpr int kTsThreads = 256;
+constexpr long long kTsMaxDim = 1024;
+template <typename T>
+__global__ void __launch_bounds__(kTsThreads)
+k_trl_steps(const __grid_constant__ HvJobT<T> jb, const ModelDev *__restrict__ mdl, const __grid_constant__ VPtrs<T> V,
+            const T *start, int k, int ncv, int ld, double *__restrict__ Hp, int ldh)
+{
+    constexpr int NT = kTsThreads, NWARP = NT / 32;
+    extern __shared__ double raw[];
+    const int nimp = mdl->nimp, npair = mdl->npair, nu = jb.nu, nd = jb.nd, n = nu * nd;
+    T *const xs = (T *)raw, *const ws = xs + n;
+    int *const at = (int *)(ws + n);
+    __shared__ T s_cross[kMaxImp * kMaxImp];
+    __shared__ unsigned s_pmask[kMaxImp];
+    __shared__ int s_t4[kMaxPair * kMaxImp];
+    __shared__ double s_h[2][kTrlMaxNcv + 1], s_red[32], s_sc[2];
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    for (int i = tid; i < npair * nimp; i += NT) s_t4[i] = mdl->t4[i];
+    for (int i = tid; i < nimp; i += NT) s_pmask[i] = mdl->pairmask[i];
+    for (int i = tid; i < nimp * nimp; i += NT) s_cross[i] = (T)mdl->cross[i];
+    for (int d = wid; d < nd; d += NWARP)
+        for (int u = lane; u < nu; u += 32) at[d * nu + u] = d * ld + u;
+    const T Jc = (T)mdl->J;
+    __syncthreads();
+    // ||w|| and its inverse, fixed order
+    const auto norm = [&] {
+        double a = 0.0;
+        for (int i = tid; i < n; i += NT) {
+            const double v = widen(ws[i]);
+            a = fma(v, v, a);
+        }
+        a = block_sum(a, s_red);
+        if (tid == 0) {
+            const double inv = a > 0.0 ? rsqrt_pos(a) : 0.0;
+            s_sc[0] = a > 0.0 ? a * inv : a;
+            s_sc[1] = inv;
+        }
+        __syncthreads();
+    };
+    // xs = w / ||w||, and to global memory with zero pads
+    const auto put = [&](T *v) {
+        const T s = (T)s_sc[1];
+        for (int i = tid; i < n; i += NT) v[at[i]] = xs[i] = ws[i] * s;
+        for (int d = wid; d < nd; d += NWARP)
+            for (int u = nu + lane; u < ld; u += 32) v[d * ld + u] = T(0);
+        __syncthreads();
+    };
+    if (start) {
+        for (int i = tid; i < n; i += NT) ws[i] = start[at[i]];
+        __syncthreads();
+        norm();
+        put(const_cast<T *>(V.p[k]));
+    } else {
+        for (int i = tid; i < n; i += NT) xs[i] = V.p[k][at[i]];
+        __syncthreads();
+    }
+    for (int j = k; j < ncv; ++j) {
+        for (int i = tid; i < n; i += NT) {
+            const int d = i / nu, u = i - d * nu, inf = __ldg(jb.up_info + u), dinf = __ldg(jb.dn_info + d);
+            const T diag = __ldg(jb.up_diag + u) + __ldg(jb.dn_diag + d) +
+                           s_cross[((inf >> 8) & 0xff) * nimp + ((dinf >> 8) & 0xff)];
+            ws[i] = hv_moves<T, T, false>(jb, mdl, xs, d, u, inf, dinf, s_pmask, s_t4, nimp, Jc, diag * xs[i]);
+        }
+        __syncthreads();
+#pragma unroll 1
+        for (int pass = 0; pass < 2; ++pass) {
+            for (int l = wid; l <= j; l += NWARP) {
+                const T *v = V.p[l];
+                T s = T(0);
+                for (int i = lane; i < n; i += 32) s += v[at[i]] * ws[i];
+                s = warp_sum(s);
+                if (lane == 0) s_h[pass][l] = widen(s);
+            }
+            __syncthreads();
+            for (int i = tid; i < n; i += NT) {
+                T w = ws[i];
+#pragma unroll 4
+                for (int l = 0; l <= j; ++l) w -= (T)s_h[pass][l] * V.p[l][at[i]];
+                ws[i] = w;
+            }
+            __syncthreads();
+        }
+        norm();
+        for (int l = tid; l <= j; l += NT) Hp[(size_t)j * ldh + l] = s_h[0][l] + s_h[1][l];
+        if (tid == 0) Hp[(size_t)j * ldh + j + 1] = s_sc[0];
+        if (j + 1 >= n) break;
+        put(const_cast<T *>(V.p[j + 1]));
+    }
+}
+
 template <typename T>
 static int trl_solve(mo_ed_ctx *ctx, const Sector &s, int nev, std::vector<double> &vals,
                      std::vector<DevBuf> *vecs)
@@ -626,11 +725,21 @@ static int trl_solve(mo_ed_ctx *ctx, const Sector &s, int nev, std::vector<doubl
         return MO_ED_OK;
     };
 
+    // small sectors: a cycle's steps in one launch
+    HvJobT<T> job;
+    bool small = false;
+    if (D <= kTsMaxDim) {
+        if (int rc = hv_row_job<T>(ctx, s, kind, &job, &small)) return rc;
+        job.ld = job.nu;
+    }
+
     // start vector
     unsigned long long seed = 0x5eedULL + 977ULL * (unsigned)s.ne_up + 131ULL * (unsigned)s.ne_down;
     k_random<T><<<G, kVecThreads, 0, ctx->stream>>>((T *)W->p, Dp, s.ld(), s.up->n, seed);
     MOED_CHECK_LAUNCH(ctx);
-    if (int rc = normalize_into((T *)W->p, V[0])) return rc;
+    const T *start = small ? (const T *)W->p : nullptr;
+    if (!small)
+        if (int rc = normalize_into((T *)W->p, V[0])) return rc;
 
     int k = 0;           // kept Ritz vectors at the front of V
     int m = ncv;
@@ -644,7 +753,15 @@ static int trl_solve(mo_ed_ctx *ctx, const Sector &s, int nev, std::vector<doubl
         // the betas are read once at the end of the cycle.  A step whose beta
         // falls below the breakdown threshold ends the cycle there (its Krylov
         // space is invariant; later steps of the cycle are discarded).
-        for (int j = k; j < ncv; ++j) {
+        if (small) {
+            m = (int)std::min<long long>(ncv, D);
+            k_trl_steps<T><<<1, kTsThreads, (2 * sizeof(T) + sizeof(int)) * (size_t)D, ctx->stream>>>(
+                job, ctx->d_mdl, make_ptrs<T>(V, ncv + 1), start, k, ncv, s.ld(), Hp, ldh);
+            MOED_CHECK_LAUNCH(ctx);
+            matvecs += m - k;
+            start = nullptr;
+        }
+        for (int j = small ? ncv : k; j < ncv; ++j) {
             if (int rc = hv(V[j]->p, W->p)) return rc;
             const bool last = j + 1 >= D;   // Krylov space is the whole sector
             OrthoCoef oc;

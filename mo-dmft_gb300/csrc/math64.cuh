@@ -33,6 +33,22 @@ __device__ __forceinline__ double rcp_pos(double d)
     return fma(y0, fma(e, e, e), y0);
 }
 
+__device__ __forceinline__ double widen(float f);
+
+// 1/sqrt(d) for d > 0: an FP32 seed y0 of rsqrt.approx refined by one step of
+// the binomial series
+//   (1 - e)^(-1/2) = 1 + e (1/2 + 3/8 e) + O(e^3),  e = 1 - d y0^2, |e| < 2^-20,
+// five dependent FP64 instructions where a square root and a division take
+// tens.  Outside [2^-100, 2^100] (and for d <= 0, non-finite d) it is those.
+__device__ __forceinline__ double rsqrt_pos(double d)
+{
+    if ((unsigned)((int)(__double_as_longlong(d) >> 52) - 923) > 200u) return 1.0 / sqrt(d);
+    float yf;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(yf) : "f"((float)d));
+    const double y0 = widen(yf), e = fma(-(d * y0), y0, 1.0);
+    return fma(y0 * e, fma(e, 0.375, 0.5), y0);
+}
+
 // (double)f by integer operations: a conversion instruction takes a slot of
 // the FP64 pipe, even one that is predicated off, so the rare cases have none
 // either.  Infinities and NaN need the exponent 2047 instead of 255 + 896; a

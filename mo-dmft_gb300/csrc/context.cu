@@ -32,6 +32,11 @@ int dev_alloc(mo_ed_ctx *ctx, DevBuf &b, size_t bytes)
     b.release();
     if (bytes == 0) bytes = 16;
     cudaError_t e = cudaMalloc(&b.p, bytes);
+    if (e == cudaErrorMemoryAllocation && !ctx->kry_busy && !ctx->kry_pool.empty()) {
+        cudaGetLastError();
+        ctx->kry_pool.clear();   // the Krylov vectors kept between solves
+        e = cudaMalloc(&b.p, bytes);
+    }
     if (e != cudaSuccess) {
         b.p = nullptr;
         cudaGetLastError();
@@ -43,12 +48,28 @@ int dev_alloc(mo_ed_ctx *ctx, DevBuf &b, size_t bytes)
 
 int dev_alloc_slab(mo_ed_ctx *ctx, DevBuf *b, int n, size_t bytes)
 {
-    const size_t step = (bytes + 255) & ~(size_t)255;
-    DevBuf all;
-    if (int rc = dev_alloc(ctx, all, step * (size_t)n)) return rc;
-    std::shared_ptr<void> own(all.p, [](void *q) { cudaFree(q); });
-    char *base = (char *)all.p;
-    all.p = nullptr;
+    // small sets of several calls share an allocation of kSlabShare (90 us
+    // each otherwise, when several threads allocate)
+    constexpr size_t kSlabShare = (size_t)2 << 20;
+    const size_t step = (bytes + 255) & ~(size_t)255, need = step * (size_t)n;
+    std::shared_ptr<void> own;
+    char *base;
+    if (ctx->slab && ctx->slab_used + need <= kSlabShare) {
+        own = ctx->slab;
+        base = (char *)own.get() + ctx->slab_used;
+        ctx->slab_used += need;
+    } else {
+        DevBuf all;
+        const bool share = need <= kSlabShare / 2;
+        if (int rc = dev_alloc(ctx, all, share ? kSlabShare : need)) return rc;
+        own = std::shared_ptr<void>(all.p, [](void *q) { cudaFree(q); });
+        base = (char *)all.p;
+        all.p = nullptr;
+        if (share) {
+            ctx->slab = own;
+            ctx->slab_used = need;
+        }
+    }
     for (int i = 0; i < n; ++i) {
         b[i].release();
         b[i].p = base + step * (size_t)i;

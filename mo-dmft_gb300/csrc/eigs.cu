@@ -47,7 +47,11 @@ namespace cg = cooperative_groups;
 constexpr int kKryMax = 352;                           // Krylov vectors of one run
 constexpr size_t kKryRunBytes = (size_t)48 << 30;      // and their memory (at most half of what is free)
 constexpr long long kKryMinDim = 128;                  // smaller sectors: thick restarts (krylov.cu)
-constexpr size_t kKryPoolBytes = (size_t)4 << 30;      // Krylov vectors kept in the context between solves
+// Krylov vectors kept in the context between solves: up to the first without
+// asking; up to the second (not in the worker contexts of a solve) while that is
+// at most a quarter of the free memory.  20 GB of an eigensolve of 15 million
+// FP32 elements: 10 ms to allocate in 240 MB chunks and 17 ms to free, of 150.
+constexpr size_t kKryPoolBytes = (size_t)4 << 30, kKryKeepBytes = (size_t)24 << 30;
 constexpr size_t kRrPoolBytes = (size_t)64 << 20;      // largest FP64 vector of the pooled Rayleigh-Ritz workspace
 constexpr size_t kSlabBytes = (size_t)1 << 20;         // returned vectors up to this size share one allocation
 // k_kry_cluster: sectors up to these sizes, shared memory of a CTA.  4 states
@@ -570,22 +574,40 @@ struct KryVectors {
     mo_ed_ctx *ctx;
     size_t vb;
     int per;                             // vectors per chunk
-    bool pooled;
-    std::vector<DevBuf> local;
+    std::vector<DevBuf> local;           // chunks past those of the context's pool
     std::vector<void *> p;               // vector j
-    int chunks = 0;
-    KryVectors(mo_ed_ctx *c, size_t bytes, int most) : ctx(c), vb((bytes + 255) & ~(size_t)255)
+    size_t chunks = 0;
+    bool pooled = true;
+    KryVectors(mo_ed_ctx *c, size_t bytes) : ctx(c), vb((bytes + 255) & ~(size_t)255)
     {
-        per = (int)std::max<size_t>(1, std::min<size_t>(32, ((size_t)256 << 20) / vb));
-        pooled = vb * (size_t)(most + per) <= kKryPoolBytes;
+        per = (int)std::max<size_t>(1, std::min<size_t>(32, ((size_t)1 << 30) / vb));
+        ctx->kry_busy = true;
+    }
+    ~KryVectors() { ctx->kry_busy = false; }
+    KryVectors(const KryVectors &) = delete;
+    // whether the pool may hold `bytes` in chunk i
+    bool keeps(size_t i, size_t bytes) const
+    {
+        size_t total = bytes;
+        for (size_t k = 0; k < ctx->kry_pool.size(); ++k)
+            if (k != i) total += ctx->kry_pool[k].bytes;
+        if (total <= kKryPoolBytes) return true;
+        if (ctx->worker || total > kKryKeepBytes) return false;
+        size_t fr = 0, tot = 0;
+        return cudaMemGetInfo(&fr, &tot) == cudaSuccess && total <= fr / 4;
     }
     int grow(int n)                      // vectors 0 .. n-1 exist
     {
-        std::vector<DevBuf> &store = pooled ? ctx->kry_pool : local;
         while ((int)p.size() < n) {
-            if ((int)store.size() <= chunks) store.resize(chunks + 1);
-            if (int rc = ensure(ctx, store[chunks], vb * per)) return rc;
-            for (int i = 0; i < per; ++i) p.push_back((char *)store[chunks].p + vb * i);
+            const size_t need = vb * (size_t)per;
+            if (pooled) {
+                if (ctx->kry_pool.size() <= chunks) ctx->kry_pool.resize(chunks + 1);
+                pooled = ctx->kry_pool[chunks].bytes >= need || keeps(chunks, need);
+            }
+            if (!pooled) local.emplace_back();
+            DevBuf &b = pooled ? ctx->kry_pool[chunks] : local.back();
+            if (int rc = ensure(ctx, b, need)) return rc;
+            for (int i = 0; i < per; ++i) p.push_back((char *)b.p + vb * i);
             ++chunks;
         }
         return MO_ED_OK;
@@ -634,7 +656,7 @@ struct KryRun {
 
     KryRun(mo_ed_ctx *c, const Sector &sec, int nw, int most, int lo, double tl)
         : ctx(c), s(sec), nwant(nw), mmax(most), least(lo), tol(tl), Dp(sec.Dpad()), vb(sizeof(T) * (size_t)sec.Dpad()),
-          kind(f32 ? HV_F32 : HV_F64), U(c, sizeof(T) * (size_t)sec.Dpad(), most + 2), al(ns), be(ns), inv(ns), th(nw),
+          kind(f32 ? HV_F32 : HV_F64), U(c, sizeof(T) * (size_t)sec.Dpad()), al(ns), be(ns), inv(ns), th(nw),
           y(ns)
     {
         G = (int)std::max(1LL, std::min((Dp / 4 + kVecThreads - 1) / kVecThreads, (long long)ctx->num_sms * 8));
@@ -1174,6 +1196,7 @@ int plz_solve(mo_ed_ctx *ctx, const Sector &s, int nev, std::vector<double> &val
     if (vb * (size_t)mmax > kKryPoolBytes) {
         size_t fr = 0, tot = 0;
         MOED_CUDA(ctx, cudaMemGetInfo(&fr, &tot));
+        for (const DevBuf &b : ctx->kry_pool) fr += b.bytes;
         mmax = (int)std::min<size_t>(mmax, std::min(kKryRunBytes, fr / 2) / vb);
         if (mmax < least + 40) return MO_ED_OK;
     }

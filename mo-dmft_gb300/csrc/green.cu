@@ -637,6 +637,7 @@ static int solve_sectors(mo_ed_ctx *ctx, int nev, std::vector<double> &eig_all,
     while ((int)ctx->workers.size() < nthreads) {
         mo_ed_ctx *w = nullptr;
         if (int rc = mo_ed_create(&w, ctx->device, nullptr)) return fail(ctx, rc, "worker context");
+        w->worker = true;
         ctx->workers.push_back(w);
         ctx->worker_gen.push_back(-1);
     }

@@ -294,10 +294,14 @@ struct mo_ed_ctx {
     // eigensolver workspace reused across sectors (Krylov vectors of sectors
     // up to 64 MB per vector, and the projected-problem arrays)
     std::vector<moed::DevBuf> trl_pool, trl_small, rr_pool;
-    // eigs.cu: chunks of Krylov vectors kept between solves (at most
-    // kKryPoolBytes together), small arrays, and pinned host memory for the
+    // eigs.cu: chunks of Krylov vectors kept between solves (KryVectors; given
+    // back when an allocation fails while no run uses them), small arrays, and pinned host memory for the
     // coefficients read while the next steps run
     std::vector<moed::DevBuf> kry_pool, kry_small;
+    bool kry_busy = false, worker = false;
+    // where the next small returned vectors go (dev_alloc_slab)
+    std::shared_ptr<void> slab;
+    size_t slab_used = 0;
     moed::DevBuf lz_pool;      // workspace of lanczos_iteration and the Green's function, up to kLzPoolBytes
     void *pinned = nullptr;
     size_t pinned_bytes = 0;

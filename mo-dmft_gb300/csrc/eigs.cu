@@ -908,7 +908,10 @@ struct KryRun {
         hmax = anorm = 0.0;
         const double unit = f32 ? 6e-8 : 1.1e-16;
         const double target = f32 ? 2e-5 : 1e-11, most_h = f32 ? 1e-2 : 1e-4;
-        int pmax = f32 ? 16 : 24;
+        // The longest period rises while little is found.  In small sectors, where
+        // a reorthogonalisation costs about a step, it does not: one that comes
+        // too late costs a period's steps.  9 million FP32 elements: 79 -> 65 ms.
+        int pmax = f32 ? 16 : 24, ptop = s.D() < (1 << 19) ? pmax : 2 * pmax;
         int judged = -1, good = -1;   // last reorthogonalisation judged, and found small
         double grow = 0.0;            // largest growth per step seen
         double last_res = 0.0;
@@ -956,7 +959,7 @@ struct KryRun {
                     // orthogonality was lost before this reorthogonalisation:
                     // back to the last one known to be good, shorter periods
                     if (good < 0 || read_gap[slot] <= 2) return MO_ED_OK;
-                    pmax = period = std::max(2, std::min(read_gap[slot], pmax) / 2);
+                    ptop = pmax = period = std::max(2, std::min(read_gap[slot], pmax) / 2);
                     if (int rc = go_back(good)) return rc;
                     j = good + 1;
                     full = false;
@@ -967,8 +970,12 @@ struct KryRun {
                     continue;
                 }
                 judged = good = jr;
+                // Components c taken out once leave c^2 in every vector to come (the
+                // earlier vectors are orthogonal to c only), which does not grow.
+                const int gap = read_gap[slot];
+                grow = std::max(grow, std::max(std::log(c / std::max(2 * unit, hmax * hmax)), 0.3) / gap);
                 hmax = std::max(hmax, c);
-                grow = std::max(grow, std::max(std::log(c / (2 * unit)), 0.3) / read_gap[slot]);
+                if (c < target) pmax = std::max(pmax, std::min(ptop, gap + gap / 4 + 1));
                 period = std::max(2, std::min(base > 0 ? std::min(5, pmax) : pmax, (int)(std::log(target / (2 * unit)) / grow)));
             }
             const double want = tol * std::max(anorm, 1.0);

@@ -82,9 +82,13 @@ __host__ __device__ inline size_t chi2_smem_bytes(int nx, int nbath, int nt)
            sizeof(int) * (kMaxOrb * kListMax + kMaxOrb);
 }
 
-__device__ __forceinline__ bool finite_bits(double x)
+__host__ __device__ __forceinline__ bool finite_bits(double x)
 {
+#ifdef __CUDA_ARCH__
     return ((__double_as_longlong(x) >> 52) & 0x7ff) != 0x7ff;
+#else
+    return std::isfinite(x);
+#endif
 }
 
 // Sums of the chi^2 terms of one parameter set xb (shared or global memory)
@@ -222,6 +226,137 @@ __device__ void chi2_sums(const double *__restrict__ xb, int nx, bool grad, int 
             out[1 + i] = ((red[4 * i] + red[4 * i + 1]) + red[4 * i + 2]) + red[4 * i + 3];
     }
     if (final_sync) __syncthreads();
+}
+
+// A thread's w_n are the same for every evaluation of a fit, so what an
+// evaluation takes from omega and D_ev is laid out once per launch: for the
+// first nstage of them wz, wz^2, 1 / w_n and D_ev per orbital, [nstage][3 + 2
+// norb][nt].
+struct FitStage {
+    double *p;
+    int n;
+};
+__host__ __device__ inline size_t fit_stage_doubles(int nstage, int norb, int nt)
+{
+    return (size_t)nstage * (3 + 2 * norb) * nt;
+}
+__device__ __forceinline__ void fit_stage_fill(const FitStage &st, int nw, int n_first, int n_step, int norb,
+                                               const double *__restrict__ omega, const double *__restrict__ dev, int fcmplx)
+{
+    const int tid = threadIdx.x, nt = blockDim.x;
+    for (int i = 0; i < st.n; ++i) {
+        const int n = n_first + tid + i * n_step;
+        if (n >= nw) break;
+        double *s = st.p + (size_t)i * (3 + 2 * norb) * nt + tid;
+        const double w = omega[n], wz = fcmplx ? (double)(float)w : w;
+        s[0] = wz;
+        s[nt] = wz * wz;
+        s[2 * nt] = rcp_pos(w);
+        for (int a = 0; a < 2 * norb; ++a) s[(size_t)(3 + a) * nt] = dev[2 * (size_t)n * norb + a];
+    }
+}
+
+// 1/z_k of N levels from k0 into the thread's column of sz (chi2_sums)
+template <int N>
+__device__ __forceinline__ void fit_levels(const double *eps, int k0, double wz, double wz2, double *sz, int nt)
+{
+    double d[N], y[N];
+#pragma unroll
+    for (int i = 0; i < N; ++i) d[i] = fma(eps[k0 + i], eps[k0 + i], wz2);
+    rcp_pos_n<N>(d, y);
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        sz[(size_t)(2 * (k0 + i)) * nt] = -eps[k0 + i] * y[i];
+        sz[(size_t)(2 * (k0 + i) + 1) * nt] = -wz * y[i];
+    }
+}
+
+// chi2_sums' lists of the couplings at xb, by one warp
+__device__ __forceinline__ void fit_lists(const double *xb, int nx, int norb, int nbath, double *sm)
+{
+    const int nt = blockDim.x, lane = threadIdx.x & 31;
+    double *lv2 = sm + (size_t)nx * nt + 2 * (size_t)nbath * nt + kRedSlots;
+    int *lk = (int *)(lv2 + 2 * kMaxOrb * kListMax);
+    int *lcnt = lk + kMaxOrb * kListMax;
+    const bool eps_ok = lane < nbath && finite_bits(xb[lane]);
+    for (int a = 0; a < norb; ++a) {
+        const double v = lane < nbath ? xb[nbath + a * nbath + lane] : 0.0;
+        const bool keep = lane < nbath && ((__double_as_longlong(v) << 1) != 0 || !eps_ok);
+        const unsigned m = __ballot_sync(0xffffffffu, keep);
+        if (keep) {
+            const int c = __popc(m & ((1u << lane) - 1u));
+            lk[a * kListMax + c] = lane;
+            lv2[a * kListMax + c] = v * v;
+        }
+        if (lane == 0) lcnt[a] = __popc(m);
+    }
+}
+
+// FUNC's sum at xb for the line search of a fit: the terms and the order of
+// chi2_sums (whose lists fit_lists has made), the partial sum of each warp left in
+// slot[rank][warp] of every CTA of the cluster (lane r writes rank r's).  An evaluation is a chain of
+// latencies (one w_n per thread): 8,050 cycles in chi2_sums at 1 x 4, 1,024
+// w_n; 5,800 here (lists 700, levels 2,900, residual 1,600, warp sums 600), with
+// the constants of the w_n laid out beforehand and the levels' reciprocals
+// interleaved.  Sharing the sums takes 3,100 more (3,500), the line search's own
+// arithmetic 4,500.
+__device__ __forceinline__ void fit_func_sum(const double *xb, int nx, int nw, int n_first, int n_step, int norb, int nbath,
+                                             const double *__restrict__ omega, const double *__restrict__ dev, int fcmplx,
+                                             double *sm, const FitStage &st, double *slot, int rank, int ncta)
+{
+    const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, wid = tid >> 5;
+    double *sz = sm + (size_t)nx * nt;                 // as in chi2_sums
+    const double *lv2 = sz + 2 * (size_t)nbath * nt + kRedSlots;
+    const int *lk = (const int *)(lv2 + 2 * kMaxOrb * kListMax), *lcnt = lk + kMaxOrb * kListMax;
+    const double *eps = xb, *ef = xb + nx - norb;
+    double fsum = 0.0;
+    for (int i = 0, n = n_first + tid; n < nw; ++i, n += n_step) {
+        double wz, wz2, inv_w;
+        const double *D;
+        int ds;
+        if (i < st.n) {
+            const double *s = st.p + (size_t)i * (3 + 2 * norb) * nt + tid;
+            wz = s[0];
+            wz2 = s[nt];
+            inv_w = s[2 * nt];
+            D = s + 3 * nt;
+            ds = nt;
+        } else {
+            const double w = omega[n];
+            wz = fcmplx ? (double)(float)w : w;
+            wz2 = wz * wz;
+            inv_w = rcp_pos(w);
+            D = dev + 2 * (size_t)n * norb;
+            ds = 1;
+        }
+        int k = 0;
+        for (; k + 4 <= nbath; k += 4) fit_levels<4>(eps, k, wz, wz2, sz + tid, nt);
+        if (k + 2 <= nbath) {
+            fit_levels<2>(eps, k, wz, wz2, sz + tid, nt);
+            k += 2;
+        }
+        if (k < nbath) fit_levels<1>(eps, k, wz, wz2, sz + tid, nt);
+        for (int a = 0; a < norb; ++a) {
+            double dre = 0.0, dim = 0.0;
+            const int cnt = lcnt[a];
+#pragma unroll 4
+            for (int j = 0; j < cnt; ++j) {
+                const int kk = lk[a * kListMax + j];
+                const double v2 = lv2[a * kListMax + j];
+                dre = fma(v2, sz[(size_t)(2 * kk) * nt + tid], dre);
+                dim = fma(v2, sz[(size_t)(2 * kk + 1) * nt + tid], dim);
+            }
+            const double rr = (dre + ef[a]) - D[(size_t)(2 * a) * ds], ri = dim - D[(size_t)(2 * a + 1) * ds];
+            fsum = fma(fma(rr, rr, ri * ri), inv_w, fsum);
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) fsum += __shfl_xor_sync(0xffffffffu, fsum, o);
+    if (ncta == 1) {
+        if (lane == 0) slot[wid] = fsum;
+    } else if (lane < ncta) {
+        cg::this_cluster().map_shared_rank(slot, lane)[rank * (nt >> 5) + wid] = fsum;
+    }
 }
 
 // FUNC = sum / (norb^2 nw) (func.f90:40-43) from out[0] of chi2_sums over
@@ -441,14 +576,6 @@ __global__ void k_calc_dev(int norb, int nbath, int nw, const double *omega, con
     dev[2 * (size_t)t + 1] = d.y;
 }
 
-// dynamic shared memory of k_chi2 / k_fit for these dimensions and nt threads
-static int chi2_smem(mo_ed_ctx *ctx, const void *kernel, int nx, int nbath, int nt, size_t *bytes)
-{
-    *bytes = chi2_smem_bytes(nx, nbath, nt);
-    MOED_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)*bytes));
-    return MO_ED_OK;
-}
-
 // k_chi2 over nbatch sets.  A set is split over 2, 4, 8 CTAs while threads
 // have more than one w_n and, for 4 and 8, every CTA finds an SM of its own
 // (larger clusters two to an SM leave a part wave).  3 x 12, 512 w_n, 1 / 2 /
@@ -564,11 +691,12 @@ struct Frprmn {
     // frprmn.f90:212-234: func at pcom + x xicom (formed by the functor)
     __host__ __device__ double f1dim(double x) { return func.line(pcom, xicom, x); }
 
-    __host__ __device__ void mnbrak(double &ax, double &bx, double &cx, double &fa, double &fb, double &fc)
+    // f0: f1dim(ax) where it is known, else null
+    __host__ __device__ void mnbrak(double &ax, double &bx, double &cx, double &fa, double &fb, double &fc, const double *f0)
     {
         const double GOLD = (double)1.618034f, GLIMIT = (double)100.f, TINY = (double)1.e-20f;
         double dum, fu, q, r, u, ulim;
-        fa = f1dim(ax);
+        fa = f0 ? *f0 : f1dim(ax);
         fb = f1dim(bx);
         if (fb > fa) {
             dum = ax; ax = bx; bx = dum;
@@ -611,7 +739,8 @@ struct Frprmn {
         }
     }
 
-    __host__ __device__ int brent(double ax, double bx, double cx, double tol, double &xmin, double &fret)
+    // fbx: f1dim(bx), which mnbrak has left
+    __host__ __device__ int brent(double ax, double bx, double cx, double fbx, double tol, double &xmin, double &fret)
     {
         const int ITMAX = 100;
         const double CGOLD = (double).3819660f, ZEPS = (double)1.0e-10f;
@@ -620,7 +749,7 @@ struct Frprmn {
         b = fmax(ax, cx);
         v = bx; w = v; x = v;
         e = 0.;
-        fx = f1dim(x);
+        fx = fbx;
         fv = fx; fw = fx;
         for (int iter = 1; iter <= ITMAX; ++iter) {
             xm = 0.5 * (a + b);
@@ -671,20 +800,23 @@ struct Frprmn {
         return MO_ED_ERR_FIT;
     }
 
-    __host__ __device__ int linmin(double *p, double *xi, double &fret)
+    // fp0: the function at p where it is known, else null (p + 0 xi = p then,
+    // unless an element of xi is not finite)
+    __host__ __device__ int linmin(double *p, double *xi, double &fret, const double *fp0)
     {
         const double TOL = (double)1.e-8f;
         double pc[kMaxX], xc[kMaxX], ax, xx, bx, fa, fx, fb, xmin = 0.0;
         for (int j = 0; j < n; ++j) {
             pc[j] = p[j];
             xc[j] = xi[j];
+            if (!finite_bits(xi[j])) fp0 = nullptr;
         }
         pcom = pc;
         xicom = xc;
         ax = 0.;
         xx = 1.;
-        mnbrak(ax, xx, bx, fa, fx, fb);
-        int rc = brent(ax, xx, bx, TOL, xmin, fret);
+        mnbrak(ax, xx, bx, fa, fx, fb, fp0);
+        int rc = brent(ax, xx, bx, fx, TOL, xmin, fret);
         for (int j = 0; j < n; ++j) {
             xi[j] = xmin * xi[j];
             p[j] = p[j] + xi[j];
@@ -706,13 +838,15 @@ struct Frprmn {
     {
         const int itmax = 20000;
         const double eps = 1.e-10;
-        double xi[kMaxX], dgg, gam, gg;
+        double xi[kMaxX], dgg, gam, gg, f0 = 0.0;   // f0: the function at p, as dfunc has it too
+        bool known = false;
         if (resume) {
             for (int j = 0; j < n; ++j) xi[j] = h[j];
         } else {
             its_done = 0;
             fp = func(p);
-            dfunc(p, xi);
+            f0 = dfunc(p, xi);
+            known = true;
             for (int j = 0; j < n; ++j) {
                 g[j] = -xi[j];
                 h[j] = g[j];
@@ -727,10 +861,11 @@ struct Frprmn {
                 return kFitSuspended;
             }
             iter = its;
-            if (int rc = linmin(p, xi, fret)) return rc;
+            if (int rc = linmin(p, xi, fret, known ? &f0 : nullptr)) return rc;
             if (2. * fabs(fret - fp) <= ftol * (fabs(fret) + fabs(fp) + eps)) return 0;
             fp = fret;
-            dfunc(p, xi);
+            f0 = dfunc(p, xi);
+            known = true;
             gg = 0.;
             dgg = 0.;
             for (int j = 0; j < n; ++j) {
@@ -774,6 +909,7 @@ struct Frprmn {
 constexpr int kFitCta = 256;
 constexpr int kFitMaxCluster = 8;
 constexpr size_t kFitSmemMax = 220 * 1024;
+constexpr int kFitStageMax = 4;
 
 
 // Scheduler words of one k_fit launch (global memory, zeroed before it):
@@ -781,6 +917,8 @@ constexpr size_t kFitSmemMax = 220 * 1024;
 // q[kQSusp] suspensions, q[kQGaveUp] picks that gave up (an internal error);
 // flag[b] = 1 while fit b is parked, its[b] its iterations done.
 constexpr int kQFresh = 0, kQParked = 1, kQSusp = 2, kQGaveUp = 3, kQWords = 4;
+// one parity's slots of DevChi2::fslots: every warp's sum and every CTA's
+constexpr int kFitSlots = kFitMaxCluster * kFitThreads / 32 + kFitMaxCluster;
 constexpr int kCmdFunc = 0, kCmdGrad = 1, kCmdYield = 2, kCmdDone = 3;
 
 __device__ __forceinline__ int ld_relaxed(int *a)
@@ -792,6 +930,9 @@ struct DevChi2 {
     int nx, nw, norb, nbath, fcmplx;
     const double *omega, *dev;
     double *sm, *sx, *sres, *slots;   // slots: [2][kMaxX + 1] of this CTA
+    double *fslots;                   // [2][kFitSlots]: every warp's sum of FUNC
+    FitStage stage;
+    double fdiv, frcp;                // norb^2 nw and its reciprocal
     int rank, ncta, par;
     int *q, nbatch;                   // scheduler words
     int *bcast;                       // [2] in this CTA's shared memory
@@ -862,14 +1003,43 @@ struct DevChi2 {
         par ^= 1;
         __syncthreads();   // sres is complete
     }
+    // chi^2 alone at the point sx; the value in every lane of warp 0.  A CTA's
+    // sum is its warps' in order, the total the CTAs' in order, as eval_body's.
+    __device__ double func_body()
+    {
+        const int nt = blockDim.x, nwarp = nt >> 5;
+        double *slot = fslots + par * kFitSlots;
+        fit_func_sum(sx, nx, nw, rank * nt, ncta * nt, norb, nbath, omega, dev, fcmplx, sm, stage, slot, rank, ncta);
+        par ^= 1;
+        sync_all();
+        if (threadIdx.x >= 32) return 0.0;
+        double *tot = slot + kFitMaxCluster * kFitThreads / 32;
+        if (threadIdx.x < ncta) {
+            const double *w = slot + threadIdx.x * nwarp;   // nwarp = 4 or 8; the sums are >= 0, so 0 + w[0] = w[0]
+            double s = ((w[0] + w[1]) + w[2]) + w[3];
+            if (nwarp == 8) s = (((s + w[4]) + w[5]) + w[6]) + w[7];
+            tot[threadIdx.x] = s;
+        }
+        __syncwarp();
+        double v[kFitMaxCluster];
+#pragma unroll
+        for (int r = 0; r < kFitMaxCluster; ++r) v[r] = tot[r];
+        double s = v[0];
+        if (ncta >= 2) s += v[1];
+        if (ncta >= 4) s = (s + v[2]) + v[3];
+        if (ncta == 8) s = (((s + v[4]) + v[5]) + v[6]) + v[7];
+        return div_by(s, fdiv, frcp);
+    }
     // warps 1 .. of the CTA: run the commands of warp 0 until kCmdDone
     __device__ void serve()
     {
         for (;;) {
             __syncthreads();
             const int cmd = *s_cmd;
-            if (cmd == kCmdFunc || cmd == kCmdGrad)
-                eval_body(cmd == kCmdGrad);
+            if (cmd == kCmdFunc)
+                func_body();
+            else if (cmd == kCmdGrad)
+                eval_body(true);
             else if (cmd == kCmdYield)
                 yield_body();
             else
@@ -886,10 +1056,15 @@ struct DevChi2 {
     // chi^2 (and the gradient into g) at the point sx, already in shared memory
     __device__ double eval_sx(double *g)
     {
-        command(g ? kCmdGrad : kCmdFunc);
-        eval_body(g != nullptr);
-        if (g)
-            for (int j = 0; j < nx; ++j) g[j] = sres[1 + j];
+        if (!g) {
+            __syncwarp();
+            fit_lists(sx, nx, norb, nbath, sm);
+            command(kCmdFunc);
+            return func_body();
+        }
+        command(kCmdGrad);
+        eval_body(true);
+        for (int j = 0; j < nx; ++j) g[j] = sres[1 + j];
         return sres[0];
     }
     __device__ double eval(const double *x, double *g)
@@ -912,7 +1087,7 @@ struct DevFunc {
 };
 struct DevDFunc {
     DevChi2 *c;
-    __device__ void operator()(const double *x, double *g) const { c->eval(x, g); }
+    __device__ double operator()(const double *x, double *g) const { return c->eval(x, g); }
 };
 
 // A parked fit, taken by one cluster: the one with the fewest iterations
@@ -961,15 +1136,20 @@ template <int NT, int MINB>
 __global__ void __launch_bounds__(NT, MINB)
 k_fit(double *__restrict__ X, int nbatch, int nx, int nw, int norb, int nbath, const double *__restrict__ omega,
       const double *__restrict__ dev, int fcmplx, double ftol, int ncta, int quantum, int *q, int *flag, int *its,
-      double *state, double *fret, int *iter, int *status)
+      double *state, double *fret, int *iter, int *status, int nstage, size_t stage_at)
 {
-    extern __shared__ double sm[];   // chi2_smem_bytes(nx, nbath, blockDim.x)
+    extern __shared__ double sm[];   // chi2_smem_bytes(nx, nbath, blockDim.x), then the FitStage
+    __shared__ double fslots[2 * kFitSlots];
     __shared__ double sx[kMaxX], sres[kMaxX + 1], slots[2 * (kMaxX + 1)];
     __shared__ int bcast[2], s_cmd;
     const int rank = blockIdx.x % ncta;
     const bool lead = rank == 0 && threadIdx.x == 0;
     const size_t sw = 2 * (size_t)nx + 1;
-    DevChi2 c{nx, nw, norb, nbath, fcmplx, omega, dev, sm, sx, sres, slots, rank, ncta, 0, q, nbatch, bcast, &s_cmd};
+    const FitStage stage{sm + stage_at, nstage};
+    fit_stage_fill(stage, nw, rank * blockDim.x, ncta * blockDim.x, norb, omega, dev, fcmplx);
+    const double fdiv = (double)(float)(norb * norb * nw);
+    DevChi2 c{nx, nw, norb, nbath, fcmplx, omega, dev, sm, sx, sres, slots, fslots, stage, fdiv, 1.0 / fdiv, rank, ncta, 0,
+              q, nbatch, bcast, &s_cmd};
     Frprmn<DevFunc, DevDFunc> fr{DevFunc{&c}, DevDFunc{&c}, nx};
     double p[kMaxX];
     c.sync_all();   // every CTA of the cluster runs before its shared memory is written remotely
@@ -1062,7 +1242,14 @@ static int fit_on_device(mo_ed_ctx *ctx, FitProblem &P, int nbatch, double *x, d
     if (P.nwloc < 2 * kFitThreads && chi2_smem_bytes(nx, P.nbath, kFitCta) <= kFitSmemMax) nt = kFitCta;
     size_t smem;
     auto kern = nt == kFitCta ? k_fit<kFitCta, 1> : k_fit<kFitThreads, 2>;
-    if (int rc = chi2_smem(ctx, (const void *)kern, nx, P.nbath, nt, &smem)) return rc;
+    // the FitStage of every w_n of a thread, up to kFitStageMax and the shared
+    // memory of two CTAs (kFitCta: one) per SM
+    const size_t base = chi2_smem_bytes(nx, P.nbath, nt), stage_at = (base + 15) / 16 * 2;
+    const size_t room = nt == kFitCta ? kFitSmemMax : kFitSmemMax / 2;
+    int nstage = std::min(kFitStageMax, (P.nwloc + ncta * nt - 1) / (ncta * nt));
+    while (nstage > 0 && sizeof(double) * (stage_at + fit_stage_doubles(nstage, P.norb, nt)) > room) --nstage;
+    smem = sizeof(double) * (stage_at + fit_stage_doubles(nstage, P.norb, nt));
+    MOED_CUDA(ctx, cudaFuncSetAttribute((const void *)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
     cfg.gridDim = dim3((unsigned)(nbatch * ncta));
@@ -1087,7 +1274,7 @@ static int fit_on_device(mo_ed_ctx *ctx, FitProblem &P, int nbatch, double *x, d
                                       (const double *)P.omega.p, (const double *)P.dev.p, ctx->opt.fortran_cmplx,
                                       ftol, ncta, ctx->opt.fit_quantum > 0 ? ctx->opt.fit_quantum : kFitQuantum, q,
                                       flag, its, (double *)dst.p, (double *)df.p,
-                                      (int *)di.p, (int *)ds.p));
+                                      (int *)di.p, (int *)ds.p, nstage, stage_at));
     MOED_CHECK_LAUNCH(ctx);
     int qh[kQWords];
     MOED_CUDA(ctx, cudaMemcpyAsync(x, dx.p, sizeof(double) * (size_t)nbatch * nx, cudaMemcpyDeviceToHost, ctx->stream));

@@ -33,6 +33,46 @@ __device__ __forceinline__ double rcp_pos(double d)
     return fma(y0, fma(e, e, e), y0);
 }
 
+// N of them with one look at the ranges, so that their chains of instructions
+// overlap; the same results.
+template <int N>
+__device__ __forceinline__ void rcp_pos_n(const double (&d)[N], double (&y)[N])
+{
+    bool odd = false;
+    float yf[N];
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        const long long b = __double_as_longlong(d[i]);
+        const int ex = (int)(b >> 52);
+        odd = odd || (unsigned)(ex - 898) > 250u;
+        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(yf[i]) : "f"(__int_as_float(((ex - 896) << 23) | (int)((b >> 29) & 0x7fffff))));
+    }
+    if (odd) {
+#pragma unroll 1
+        for (int i = 0; i < N; ++i) y[i] = rcp_pos(d[i]);
+        return;
+    }
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        const int fb = __float_as_int(yf[i]);
+        const double y0 = __longlong_as_double(((long long)(((fb >> 23) & 0xff) + 896) << 52) |
+                                               ((long long)(fb & 0x7fffff) << 29));
+        const double e = fma(-d[i], y0, 1.0);
+        y[i] = fma(y0, fma(e, e, e), y0);
+    }
+}
+
+// s / d, correctly rounded, with r = RN(1 / d): the last step of a division by
+// Markstein's theorem (IBM J. Res. Dev. 34, 1990), three dependent
+// instructions.  Outside the range where nothing under- or overflows it is
+// the division.
+__device__ __forceinline__ double div_by(double s, double d, double r)
+{
+    if ((unsigned)(((__double2hiint(s) >> 20) & 0x7ff) - 523) > 1000u) return s / d;   // |s| in [2^-500, 2^500]
+    const double q = s * r;
+    return fma(fma(-q, d, s), r, q);
+}
+
 __device__ __forceinline__ double widen(float f);
 
 // 1/sqrt(d) for d > 0: an FP32 seed y0 of rsqrt.approx refined by one step of

@@ -74,3 +74,25 @@ def test_chi2_batches(solver, norb, nbath, nw, nbatch, zeros):
         (fr, gr), (fa, ga) = reference(X[b], om, dev, nbath, norb)
         assert abs(f[b] - fr) <= tol * fa
         assert (abs(g[b] - gr) <= tol * ga).all()
+
+
+@pytest.mark.parametrize("norb,nbath,nw", [(1, 1, 40), (1, 2, 255), (1, 3, 256), (1, 5, 300), (2, 6, 1024), (1, 7, 2049),
+                                           (3, 6, 4096), (1, 4, 5200), (2, 4, 130)])
+def test_fit_function(solver, oracle, norb, nbath, nw):
+    """FUNC inside a fit (fit_func_sum): levels in groups of 4, 2 and 1, one
+    CTA and clusters, grids with more w_n per thread than are laid out
+    beforehand.  The value a fit returns is FUNC at the x it returns, which the
+    oracle sums in another order: 1e-12 as for FUNC itself."""
+    rng = np.random.default_rng(nbath * 100 + nw)
+    om = (2.0 * np.arange(nw) + 1.0) * np.pi / 50.0
+    solver.set_options(fortran_cmplx=True)
+    e, v = rng.uniform(-1.5, 1.5, nbath), rng.uniform(0.2, 0.5, (norb, nbath))
+    dev = (v[:, None, :] ** 2 / (1j * om[None, :, None] - e)).sum(-1) + 0.1
+    dev = dev + 1e-3 * (rng.standard_normal(dev.shape) + 1j * rng.standard_normal(dev.shape))
+    X = np.stack([np.concatenate([e + 0.02 * s, v.ravel() * (1 + 0.03 * s), np.full(norb, 0.1)]) for s in (1, -1)])
+    if norb == 2:
+        X[1, nbath] = 0.0   # a coupling that a fit keeps at zero or not, as the gradient says
+    x, f, _, _ = solver.fit_batch(X, om, dev, nbath, norb, ftol=1e-3)
+    for b in range(2):
+        fo = oracle.func(x[b], norb + nbath, om, dev, nbath, norb)
+        assert abs(f[b] - fo) < 1e-12 * fo

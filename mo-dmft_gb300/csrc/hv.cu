@@ -1646,7 +1646,10 @@ k_hv_sorted(const __grid_constant__ HvBatch<double> batch, const ModelDev *__res
         __syncthreads();
         for (int c = warp; c < jb.srt_n; c += NW) {
             const int2 h = __ldg(jb.srt_hdr + c);
-            const int uc = __ldg(jb.srt_col + 32 * c + lane), u = max(uc, 0);
+            // a lane without a column reads as lane 0 does: the 4-operator
+            // terms' partner columns exist for every column of the pattern, and
+            // not for any other
+            const int uc = __ldg(jb.srt_col + 32 * c + lane), u0 = __shfl_sync(0xffffffffu, uc, 0), u = uc >= 0 ? uc : u0;
             const int ns = h.y & 0xffff, iu = h.y >> 16;
             const unsigned *ent = jb.srt_ent + h.x + lane;
             // the loops below end by a branch: a predicated-off FP64 instruction

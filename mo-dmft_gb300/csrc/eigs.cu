@@ -60,9 +60,9 @@ constexpr size_t kSlabBytes = (size_t)1 << 20;         // returned vectors up to
 // (8 SMs' FP64 pipes are the limit there).
 constexpr long long kKcMaxDimF32 = 16384, kKcMaxDimF64 = 8192;
 constexpr int kKcSmem = 80 * 1024;
-// partial sums that the next step's blocks add themselves; with more, a
-// one-block launch does
-constexpr int kKryFuseParts = 1536;
+// partial sums that the next step's blocks add themselves (1.2 us with four warps
+// per sum and no square root); with more, a one-block launch does (6.5 us)
+constexpr int kKryFuseParts = 4096;
 
 // device scalars of a run: alpha[j] = q_j H q_j, beta[j] couples q_{j-1} and
 // q_j, inv[j] = 1 / ||U_j||
@@ -70,40 +70,22 @@ struct KryScal {
     double *alpha, *beta, *inv;
 };
 
-// fixed-order sums of a[0 .. na) (warp 0) and b[0 .. nb) (warp 1) into out[0], out[1]
-__device__ __forceinline__ void two_sums(const double *a, int na, const double *b, int nb, double *out)
-{
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    if (wid < 2) {
-        const double *p = wid ? b : a;
-        const int n = wid ? nb : na;
-        double s = 0.0;
-        for (int i = lane; i < n; i += 32) s += p[i];
-        s = warp_sum(s);
-        if (lane == 0) out[wid] = s;
-    }
-    __syncthreads();
-}
-
 // the scalars of step j from ||U_j||^2 and U_j . H U_j
 __device__ __forceinline__ void kry_store(const KryScal &sc, int j, double n2, double d)
 {
-    const double nrm = sqrt(n2);
-    sc.inv[j] = 1.0 / nrm;
-    sc.beta[j] = nrm;
-    sc.alpha[j] = d / n2;
+    const double inv = rsqrt_pos(n2);
+    sc.inv[j] = inv;
+    sc.beta[j] = n2 * inv;
+    sc.alpha[j] = d * rcp_pos(n2);
 }
 
 // the same from the partials of step j
 __global__ void __launch_bounds__(kVecThreads)
 k_kry_scalars(KryScal sc, int j, const double *__restrict__ norm_part, int gn, const double *__restrict__ dot_part, int gd)
 {
-    __shared__ double sred[32];
-    double a = 0.0, b = 0.0;
-    for (int i = threadIdx.x; i < gn; i += kVecThreads) a += norm_part[i];
-    for (int i = threadIdx.x; i < gd; i += kVecThreads) b += dot_part[i];
-    const double n2 = block_sum(a, sred), d = block_sum(b, sred);
-    if (threadIdx.x == 0) kry_store(sc, j, n2, d);
+    __shared__ double sums[10];
+    two_sums(norm_part, gn, dot_part, gd, sums);
+    if (threadIdx.x == 0) kry_store(sc, j, sums[0], sums[1]);
 }
 
 // U_j = (w - alpha_{j-1} U_{j-1}) / ||U_{j-1}|| - beta_{j-1} q_{j-2} with

@@ -160,16 +160,12 @@ __global__ void k_lz_update(const __grid_constant__ LzBatchDev b, int j)
 // (a default-REAL literal, ed_lanczos.F90:62) -- applied from j = 1 on.
 __global__ void k_lz_finalize(const __grid_constant__ LzBatchDev b, int j, int nstep)
 {
-    __shared__ double sred[32];
+    __shared__ double sums[10];
     const LzRunDev &R = b.run[blockIdx.x];
     if (*R.active == 0) return;
-    double acc = 0.0;
-    for (int i = threadIdx.x; i < R.upd_nitems; i += blockDim.x) acc += R.upd_part[i];
-    const double nrm = block_sum(acc, sred);
-    acc = 0.0;
-    for (int i = threadIdx.x; i < R.hv_nitems; i += blockDim.x) acc += R.hv_part[i];
-    const double dot = block_sum(acc, sred);
+    two_sums(R.upd_part, R.upd_nitems, R.hv_part, R.hv_nitems, sums);
     if (threadIdx.x == 0) {
+        const double nrm = sums[0], dot = sums[1];
         R.nrm[j] = nrm;
         if (j == 0 && nrm == 0.0) {        // zero start vector: no contribution
             R.a[0] = 0.0;
@@ -180,8 +176,9 @@ __global__ void k_lz_finalize(const __grid_constant__ LzBatchDev b, int j, int n
         R.a[j] = dot / nrm;
         // for the next update: square roots and divisions are tens of FP64
         // instructions, so not in its threads
-        R.inv[j] = 1.0 / sqrt(nrm);
-        R.cpl[j] = j > 0 ? sqrt(nrm / R.nrm[j - 1]) : 0.0;
+        const double inv = rsqrt_pos(nrm);
+        R.inv[j] = inv;
+        R.cpl[j] = j > 0 ? nrm * inv * R.inv[j - 1] : 0.0;
         const double tiny = (double)1.e-12f;
         if (j >= 1 && nrm < tiny) {
             *R.nstep_calc = j;

@@ -45,6 +45,26 @@ __device__ __forceinline__ double block_sum(double v, double *sred)
     return t;
 }
 
+// fixed-order sums of a[0 .. na) (warps 0-3) and b[0 .. nb) (warps 4-7) in out[0], out[1]
+// (out: 10 doubles)
+__device__ __forceinline__ void two_sums(const double *a, int na, const double *b, int nb, double *out)
+{
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const double *p = wid < 4 ? a : b;
+    const int n = wid < 4 ? na : nb;
+    double s = 0.0;
+#pragma unroll 4
+    for (int i = 32 * (wid & 3) + lane; i < n; i += 128) s += p[i];
+    s = warp_sum(s);
+    if (lane == 0) out[2 + wid] = s;
+    __syncthreads();
+    if (threadIdx.x < 2) {
+        const double *q = out + 2 + 4 * threadIdx.x;
+        out[threadIdx.x] = (q[0] + q[1]) + (q[2] + q[3]);
+    }
+    __syncwarp();   // read by thread 0
+}
+
 template <typename TX, typename TY>
 __global__ void k_dot_part(const TX *__restrict__ x, const TY *__restrict__ y, long long n,
                            double *part)

@@ -207,8 +207,9 @@ int mo_ed_lanczos_iteration_noalloc(mo_ed_ctx *ctx, int ne_up, int ne_down, cons
                                     int *nstep_calc, double *a, double *b);
 
 /* ---- a13: diag (ed_solver.F90:107-191) ---------------------------------- */
-/* nev lowest eigenpairs of one sector (thick-restart Lanczos with full
- * reorthogonalisation; FP64 Rayleigh quotients).  eigval[nev] (unconverged /
+/* nev lowest eigenpairs of one sector (a Lanczos run with periodic
+ * reorthogonalisation, thick restarts in the smallest sectors; FP64
+ * Rayleigh-Ritz).  eigval[nev] (unconverged /
  * nonexistent levels: DBL_MAX, like the reference's huge()); eigvec may be
  * NULL or a host (ntot, nev) column-major FP64 array. */
 int mo_ed_diag(mo_ed_ctx *ctx, int ne_up, int ne_down, int nev, double *eigval, double *eigvec);

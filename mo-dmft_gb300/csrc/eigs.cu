@@ -97,7 +97,7 @@ k_kry_update(KryScal sc, int j, const double *__restrict__ norm_part, int gn, co
              int gd, const T *__restrict__ w, const T *__restrict__ uc, const T *__restrict__ up, T *__restrict__ un,
              long long D, double *__restrict__ norm_out)
 {
-    __shared__ double sred[32];
+    __shared__ double sred[kVecThreads];
     __shared__ T coef[3];
     // square roots and divisions are tens of FP64 instructions: one thread's
     if (FUSED) two_sums(norm_part, gn, dot_part, gd, sred);
@@ -136,14 +136,14 @@ k_kry_update(KryScal sc, int j, const double *__restrict__ norm_part, int gn, co
         // ||U_j||^2: partials of 4 squares in T, added in FP64 every 8 iterations
         sacc += (v[0] * v[0] + v[1] * v[1]) + (v[2] * v[2] + v[3] * v[3]);
         if (++cnt == 8) {
-            acc += (double)sacc;
+            acc += widen(sacc);
             sacc = T(0);
             cnt = 0;
         }
         vstore4(un + i, v);
     }
-    acc += (double)sacc;
-    const double t = block_sum(acc, sred);
+    acc += widen(sacc);
+    const double t = block_sum_few(acc, sred);
     if (threadIdx.x == 0) norm_out[blockIdx.x] = t;
 }
 
@@ -481,8 +481,7 @@ int ritz_pairs(mo_ed_ctx *ctx, const Sector &s, const VPtrs<T> &V, int m, const 
         memset(&Xp, 0, sizeof(Xp));
         const int nc = std::min(8, nout - c0);
         for (int c = 0; c < nc; ++c) Xp.p[c] = X.p[c0 + c];
-        k_rotate<T, 8><<<G, kVecThreads, 0, ctx->stream>>>(V, m, d_Y, m, c0, nc, Xp, Dp);
-        MOED_CHECK_LAUNCH(ctx);
+        if (int rc = rotate<T>(ctx, G, V, m, d_Y, m, c0, nc, Xp, Dp)) return rc;
     }
     const int hk = sizeof(T) == 4 ? HV_MIXED : HV_F64;
     if (int rc = hv_multi(ctx, s, hk, nout, px.data(), ph.data())) return rc;
@@ -1081,8 +1080,7 @@ struct KryRun {
             memset(&O, 0, sizeof(O));
             const int nc = std::min(8, kk - c0);
             for (int c = 0; c < nc; ++c) O.p[c] = (const T *)kept[c0 + c].p;
-            k_rotate<T, 8><<<Gr, kVecThreads, 0, ctx->stream>>>(V, m, (const double *)dY.p, m, c0, nc, O, Dp);
-            MOED_CHECK_LAUNCH(ctx);
+            if (int rc = rotate<T>(ctx, Gr, V, m, (const double *)dY.p, m, c0, nc, O, Dp)) return rc;
         }
         for (int c = 0; c < kk; ++c)
             MOED_CUDA(ctx, cudaMemcpyAsync(U.p[c], kept[c].p, vb, cudaMemcpyDeviceToDevice, ctx->stream));

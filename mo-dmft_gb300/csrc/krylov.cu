@@ -113,7 +113,7 @@ __global__ void k_lz_norm0(const __grid_constant__ LzBatchDev b)
 template <typename T>
 __global__ void k_lz_update(const __grid_constant__ LzBatchDev b, int j)
 {
-    __shared__ double sred[32];
+    __shared__ double sred[kVecThreads];
     for (int item = blockIdx.x; item < b.total_items; item += gridDim.x) {
         const int r = find_run_upd(b, item);
         const LzRunDev &R = b.run[r];
@@ -144,14 +144,14 @@ __global__ void k_lz_update(const __grid_constant__ LzBatchDev b, int j)
                 v[e] = (j >= 2) ? s * (wv[e] - a * cv[e]) - c * pv[e] : s * (wv[e] - a * cv[e]);
             sacc += (v[0] * v[0] + v[1] * v[1]) + (v[2] * v[2] + v[3] * v[3]);
             if (++cnt == 8) {
-                acc += (double)sacc;
+                acc += widen(sacc);
                 sacc = T(0);
                 cnt = 0;
             }
             vstore4(un + i, v);
         }
-        acc += (double)sacc;
-        double t = block_sum(acc, sred);
+        acc += widen(sacc);
+        const double t = block_sum_few(acc, sred);
         if (threadIdx.x == 0) R.upd_part[it] = t;
     }
 }
@@ -835,8 +835,7 @@ static int trl_solve(mo_ed_ctx *ctx, const Sector &s, int nev, std::vector<doubl
             const int nc = std::min(8, kk - c0);
             std::vector<DevBuf *> outs(spare.begin() + c0, spare.begin() + c0 + nc);
             VPtrs<T> X = make_ptrs<T>(outs, nc);
-            k_rotate<T, 8><<<G, kVecThreads, 0, ctx->stream>>>(P, m, (const double *)devecs.p, m, c0, nc, X, Dp);
-            MOED_CHECK_LAUNCH(ctx);
+            if (int rc = rotate<T>(ctx, G, P, m, (const double *)devecs.p, m, c0, nc, X, Dp)) return rc;
         }
         for (int i = 0; i < kk; ++i) std::swap(V[i], spare[i]);
         if (broke) {
@@ -957,8 +956,7 @@ int refine_fp64(mo_ed_ctx *ctx, const Sector &s, const float *x, DevBuf &out, do
         VPtrs<double> P = make_ptrs<double>(V, m);
         std::vector<DevBuf *> o(1, &out);
         VPtrs<double> X = make_ptrs<double>(o, 1);
-        k_rotate<double, 8><<<G, kVecThreads, 0, ctx->stream>>>(P, m, (const double *)devecs.p, m, best, 1, X, Dp);
-        MOED_CHECK_LAUNCH(ctx);
+        if (int rc = rotate<double>(ctx, G, P, m, (const double *)devecs.p, m, best, 1, X, Dp)) return rc;
         if (*res <= 1e-9 * std::max(anorm, 1.0)) break;
     }
     return MO_ED_OK;

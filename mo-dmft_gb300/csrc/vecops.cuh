@@ -65,6 +65,25 @@ __device__ __forceinline__ void two_sums(const double *a, int na, const double *
     __syncwarp();   // read by thread 0
 }
 
+// block_sum by one warp from a buffer of kVecThreads doubles: 13 FP64 warp
+// instructions per block instead of 48, each 64 cycles of a sub-partition's
+// pipe; for kernels with a block per few elements
+__device__ __forceinline__ double block_sum_few(double v, double *buf)
+{
+    __syncthreads();
+    buf[threadIdx.x] = v;
+    __syncthreads();
+    double s[kVecThreads / 32];
+    if (threadIdx.x >= 32) return 0.0;
+#pragma unroll
+    for (int i = 0; i < kVecThreads / 32; ++i) s[i] = buf[threadIdx.x + 32 * i];
+#pragma unroll
+    for (int h = kVecThreads / 64; h; h >>= 1)
+#pragma unroll
+        for (int i = 0; i < h; ++i) s[i] += s[i + h];
+    return warp_sum(s[0]);
+}
+
 template <typename TX, typename TY>
 __global__ void k_dot_part(const TX *__restrict__ x, const TY *__restrict__ y, long long n,
                            double *part)
@@ -465,6 +484,26 @@ k_rotate(const __grid_constant__ VPtrs<T> V, int nv, const double *__restrict__ 
         for (int c = 0; c < KC; ++c)
             if (c < nc) vstore4(const_cast<T *>(X.p[c]) + i, acc[c]);
     }
+}
+
+// k_rotate of nc <= 8 columns.  FP64 is bound by its pipe, so exactly nc columns
+// (6 of 290 vectors of 0.86 million elements: 3.4 ms with 8, 2.6 with 6); FP32
+// reads at HBM speed either way.
+template <typename T>
+int rotate(mo_ed_ctx *ctx, int G, const VPtrs<T> &V, int nv, const double *Y, int ldy, int c0, int nc, const VPtrs<T> &X,
+           long long D)
+{
+    constexpr bool f64 = sizeof(T) == 8;
+    auto go = [&](auto kern) { kern<<<G, kVecThreads, 0, ctx->stream>>>(V, nv, Y, ldy, c0, nc, X, D); };
+    if (f64 && nc == 1) go(k_rotate<T, f64 ? 1 : 8>);
+    else if (f64 && nc == 2) go(k_rotate<T, f64 ? 2 : 8>);
+    else if (f64 && nc == 3) go(k_rotate<T, f64 ? 3 : 8>);
+    else if (f64 && nc == 4) go(k_rotate<T, f64 ? 4 : 8>);
+    else if (f64 && nc == 5) go(k_rotate<T, f64 ? 5 : 8>);
+    else if (f64 && nc == 6) go(k_rotate<T, f64 ? 6 : 8>);
+    else go(k_rotate<T, 8>);
+    MOED_CHECK_LAUNCH(ctx);
+    return MO_ED_OK;
 }
 
 }  // namespace moed

@@ -44,8 +44,12 @@ namespace moed {
 
 namespace cg = cooperative_groups;
 
-constexpr int kKryMax = 352;                           // Krylov vectors of one run
-constexpr size_t kKryRunBytes = (size_t)48 << 30;      // and their memory (at most half of what is free)
+// Krylov vectors of one run and their memory (at most half of what is free): a
+// run of some 350 to 480 steps restarted at 352 spends a third of its time on
+// the rotation and on steps taken again (FP64, 0.86 million elements: 413 steps, 83 -> 44 ms;
+// 41 million, 344 steps, 2.4 -> 1.3 s)
+constexpr int kKryMax = 488, kKryWide = 117;           // more vectors than kKryWide to start with: thick restarts
+constexpr size_t kKryRunBytes = (size_t)128 << 30;
 constexpr long long kKryMinDim = 128;                  // smaller sectors: thick restarts (krylov.cu)
 // Krylov vectors kept in the context between solves: up to the first without
 // asking; up to the second (not in the worker contexts of a solve) while that is
@@ -1177,7 +1181,7 @@ int plz_solve(mo_ed_ctx *ctx, const Sector &s, int nev, std::vector<double> &val
     constexpr bool f32 = sizeof(T) == 4;
     const long long D = s.D();
     const int least = 2 * nev + 24;       // vectors below which a run is not worth restarting
-    if (ctx->opt.gs_ncv > 0 || D < kKryMinDim || D < 4LL * least || least > kKryMax / 3) return MO_ED_OK;
+    if (ctx->opt.gs_ncv > 0 || D < kKryMinDim || D < 4LL * least || least > kKryWide) return MO_ED_OK;
     const double tol = ctx->opt.gs_tol > 0 ? ctx->opt.gs_tol : (f32 ? 1e-7 : 1e-11);
     const size_t vb = sizeof(T) * (size_t)s.Dpad();
     // room for the front vectors of the search below: nev

@@ -144,7 +144,7 @@ __device__ __forceinline__ void vstore4(T *p, const T (&r)[4])
     }
 }
 
-constexpr int kMaxNcv = 360;   // most vectors in one call of the kernels below
+constexpr int kMaxNcv = 496;   // most vectors in one call of the kernels below
 
 template <typename T>
 struct VPtrs {

@@ -45,9 +45,9 @@ namespace moed {
 namespace cg = cooperative_groups;
 
 // Krylov vectors of one run and their memory (at most half of what is free): a
-// run of some 350 to 480 steps restarted at 352 spends a third of its time on
-// the rotation and on steps taken again (FP64, 0.86 million elements: 413 steps, 83 -> 44 ms;
-// 41 million, 344 steps, 2.4 -> 1.3 s)
+// run of some 350 to 480 steps restarted at 352 spent half of its time on the
+// rotation and on steps taken again (FP64, 0.86 million elements, 413 steps:
+// 83 -> 44 ms; 41 million, 344 steps, 145 vectors in 48 GB: 2.4 -> 1.3 s)
 constexpr int kKryMax = 488, kKryWide = 117;           // more vectors than kKryWide to start with: thick restarts
 constexpr size_t kKryRunBytes = (size_t)128 << 30;
 constexpr long long kKryMinDim = 128;                  // smaller sectors: thick restarts (krylov.cu)

@@ -200,62 +200,14 @@ def lanczos_g_cpu(pkg, name, nev, states, matvecs, full=False, seconds=3.0):
                       f"{cfg.nstep} steps per excitation of {len(states)} kept state(s)"}
 
 
-# H*v kernel of each tile-shape variant kind (hv_tuning's fourth field)
-KERNEL_NAMES = {0: "k_hv (one row per item: k_hv_row)", 1: "k_hv_async or k_hv_wide",
-                2: "k_hv_down (128-byte slices) + k_hv_async<split>", 3: "k_hv_down (64-byte slices) + k_hv_async<split>",
-                4: "k_hv_down_rows (row AXPYs from L2) + k_hv_async<split> or k_hv_wide<split>"}
-
-
-def lanczos_g_cpu(pkg, name, nev, states, matvecs, full=False, seconds=3.0):
-    """The oracle's ed_solve + ed_calc_green_ftn on the host cores (scipy
-    ARPACK on the C restatement of multiply_H, OpenMP over rows; the
-    reference's continued-fraction Lanczos), for comparison with the device's
-    Lanczos+G of the same configuration.
-
-    full: the whole oracle path is timed.  Otherwise the time is extrapolated
-    from the oracle's H*v rate on a row sample of the first sector (about
-    `seconds` of work): (eigensolver matvecs of the device's FP64 run) x
-    t(H*v, ground sector) + nstep x sum over the excitations of the kept
-    states of t(H*v, target sector) -- H*v alone, so a lower bound."""
-    import math
-    import __graft_entry__ as g
-    O = g.load_oracle()
-    cfg = pkg.configs.config(name)
-    ek, vk = cfg.model()
-    m = O.Model(cfg.norb, cfg.nbath, cfg.U, cfg.J, ek, vk)
-    cores = os.cpu_count()
-    if full:
-        om = cfg.omega()
-        t0 = time.perf_counter()
-        st, vecs = O.ed_solve(m, cfg.sectors, nev, cfg.beta)
-        t1 = time.perf_counter()
-        O.ed_calc_green_ftn(m, cfg.sectors, st, vecs, cfg.nstep, om)
-        t2 = time.perf_counter()
-        return {"kind": "port", "mode": "full", "solve_s": round(t1 - t0, 3), "green_s": round(t2 - t1, 3),
-                "total_s": round(t2 - t0, 3), "cores": cores,
-                "sample": "oracle ed_solve (scipy ARPACK on the C multiply_H, OpenMP) + ed_calc_green_ftn, whole run"}
-    nelec, nup = cfg.sectors[0]
-    smp = cpu_baseline_sample(cfg, nup, nelec - nup, seconds)
-    t_elem = 2.0 * 8 / (smp["value"] * 1e9)           # seconds per row of H*v
-    dim = lambda nu, nd: math.comb(cfg.nsite, nu) * math.comb(cfg.nsite, nd)
-    rows = matvecs * dim(nup, nelec - nup)
-    for s in states:
-        nu_, nd_ = s["nup"], s["ndown"]
-        for ispin in ((1,) if nu_ == nd_ else (1, 2)):
-            for d in (1, -1):
-                tu, td = nu_ + (d if ispin == 1 else 0), nd_ + (d if ispin == 2 else 0)
-                if 0 <= tu <= cfg.nsite and 0 <= td <= cfg.nsite:
-                    rows += cfg.norb * cfg.nstep * dim(tu, td)
-    return {"kind": "port", "mode": "extrapolated (H*v only: a lower bound)", "total_s": round(rows * t_elem, 1),
-            "cores": cores, "hv_rows": int(rows), "rows_per_s": round(1.0 / t_elem),
-            "sample": smp["sample"] + f"; {matvecs} eigensolver matvecs (device FP64 run) + "
-                      f"{cfg.nstep} steps per excitation of {len(states)} kept state(s)"}
-
-
-# H*v kernel of each tile-shape variant kind (hv_tuning's fourth field)
-KERNEL_NAMES = {0: "k_hv", 1: "k_hv_async", 2: "k_hv_down (128-byte slices) + k_hv_async<split>",
-                3: "k_hv_down (64-byte slices) + k_hv_async<split>",
-                4: "k_hv_down_rows (row AXPYs from L2) + k_hv_async<split>"}
+def kernel_name(shape):
+    """H*v kernel of an FP32 tile shape (rows per item, threads, CTAs per SM, kind) of hv_tuning.  The shapes of
+    k_hv_wide are those of eight rows and those of four at two CTAs per SM of 512 threads."""
+    rows, threads, ctas, kind = shape
+    rest = "k_hv_wide" if rows == 8 or (rows, threads, ctas) == (4, 512, 2) else "k_hv_async"
+    return {0: "k_hv_row" if rows == 1 else "k_hv", 1: rest, 2: "k_hv_down (128-byte slices) + k_hv_async<split>",
+            3: "k_hv_down (64-byte slices) + k_hv_async<split>",
+            4: f"k_hv_down_rows (row AXPYs from L2) + {rest}<split>"}[kind]
 
 
 def lanczos_g(pkg, name, nev, precisions=("fp32", "fp32+g64", "fp64"), cpu=None):
@@ -547,7 +499,7 @@ def run_ours(args):
                     "ms_per_step": round(t_e2e * 1e3, 4)},
             "gpu_launches": launches,
             "hv_autotune": {"variants": [{"rows_per_item": v[0][0], "threads": v[0][1], "ctas_per_sm": v[0][2],
-                                          "kernel": KERNEL_NAMES[v[0][3]],
+                                          "kernel": kernel_name(v[0]),
                                           "ms": round(v[1], 4)} for v in tuning], "chosen": chosen},
             "clocks": clocks,
             "lanczos_g": lg,

@@ -36,6 +36,7 @@
 #include <cooperative_groups.h>
 
 #include "hvrow.cuh"
+#include "kryhost.h"
 #include "math64.cuh"
 #include "symeig.h"
 #include "vecops.cuh"
@@ -629,20 +630,19 @@ struct KryRun {
     unsigned long long seed = 0;
     int base = 0;                 // kept vectors of the last restart (0: none)
     int gn = 0;                   // norm partials of the last step
-    int period = 0, next_re = 0, last_re = -1;
-    struct Clean {
-        int j, gap;               // the pair (j - 1, j) was reorthogonalised, gap steps after the one before
-    };
-    std::vector<Clean> re;        // since the last restart
+    KryPeriod ctl;
+    int next_re = 0, last_re = -1;
+    std::vector<KryClean> re;     // since the last restart
+    size_t nread_re = 0;          // of them, on their way to the host
     long long matvecs = 0;
     int cycles = 0, m = 0, redo = -1;
-    double hmax = 0.0, anorm = 0.0;
+    double anorm = 0.0;
     std::vector<double> al, be, inv, th, y;
 
     KryRun(mo_ed_ctx *c, const Sector &sec, int nw, int most, int lo, double tl)
         : ctx(c), s(sec), nwant(nw), mmax(most), least(lo), tol(tl), Dp(sec.Dpad()), vb(sizeof(T) * (size_t)sec.Dpad()),
-          kind(f32 ? HV_F32 : HV_F64), U(c, sizeof(T) * (size_t)sec.Dpad()), al(ns), be(ns), inv(ns), th(nw),
-          y(ns)
+          kind(f32 ? HV_F32 : HV_F64), U(c, sizeof(T) * (size_t)sec.Dpad()), ctl(f32, sec.D()), al(ns), be(ns), inv(ns),
+          th(nw), y(ns)
     {
         // FP64: 8 elements per thread, as every block adds the last step's partials
         // on the FP64 pipe (0.86 million elements: 18.8 -> 14.4 us)
@@ -678,7 +678,7 @@ struct KryRun {
         if (int rc = ensure(ctx, sm[2], sizeof(double) * (size_t)ns * ns)) return rc;
         DevBuf &W = vb <= kRrPoolBytes ? sm[3] : wlocal;
         if (int rc = ensure(ctx, W, vb)) return rc;
-        if (int rc = ensure_pinned(ctx, sizeof(double) * 2 * 4 * ns)) return rc;
+        if (int rc = ensure_pinned(ctx, sizeof(double) * 2 * (3 + kReadRe) * ns)) return rc;
         sc.alpha = (double *)sm[0].p;
         sc.beta = sc.alpha + ns;
         sc.inv = sc.beta + 2 * ns;   // after ns doubles that hold 1 for the front vectors, read at negative offsets
@@ -746,7 +746,7 @@ struct KryRun {
             return rc;
         re.push_back({j, j - std::max(last_re, base)});
         last_re = j;
-        next_re = j + period;
+        next_re = j + ctl.period;
         return MO_ED_OK;
     }
 
@@ -851,30 +851,39 @@ struct KryRun {
         if (int rc = hv_single_dot(ctx, s, kind, U.p[j], w, dpart)) return rc;
         ++matvecs;
         while (!re.empty() && re.back().j > j) re.pop_back();
+        nread_re = re.size();
         last_re = j;
-        next_re = j + period;
+        next_re = j + ctl.period;
         redo = j + 1;
         return MO_ED_OK;
     }
 
-    // after step j: its scalars, and the components the last reorthogonalisation found, to pinned memory
-    int read_j[2], read_re[2], read_gap[2];
+    // after step j: its scalars, and the components that the reorthogonalisations
+    // since the last read have found, to pinned memory.  At most 117 steps (the
+    // first) lie between two reads, every sixth of them with one, then 44, every
+    // second; what there is no room for goes with the next read.
+    static constexpr int kReadRe = 24;
+    int read_j[2];
+    std::vector<KryClean> read_re[2];
+    double *read_at(int slot) const { return (double *)ctx->pinned + (size_t)slot * (3 + kReadRe) * ns; }
     int read_back(int slot, int j)
     {
         if (fused && !clustered) {
             k_kry_scalars<<<1, kVecThreads, 0, ctx->stream>>>(sc, j, npart[j & 1], gn, dpart, gd);
             MOED_CHECK_LAUNCH(ctx);
         }
-        double *h = (double *)ctx->pinned + (size_t)slot * 4 * ns;
+        double *h = read_at(slot);
         MOED_CUDA(ctx, cudaMemcpyAsync(h, sc.alpha, sizeof(double) * 2 * ns, cudaMemcpyDeviceToHost, ctx->stream));
         MOED_CUDA(ctx, cudaMemcpyAsync(h + 2 * ns, sc.inv, sizeof(double) * ns, cudaMemcpyDeviceToHost, ctx->stream));
-        if (last_re > 1)
-            MOED_CUDA(ctx, cudaMemcpyAsync(h + 3 * ns, hcol + (size_t)last_re * ns, sizeof(double) * ns,
-                                           cudaMemcpyDeviceToHost, ctx->stream));
+        read_re[slot].clear();
+        for (; nread_re < re.size() && read_re[slot].size() < (size_t)kReadRe; ++nread_re) {
+            h += read_re[slot].empty() ? 3 * ns : ns;
+            read_re[slot].push_back(re[nread_re]);
+            MOED_CUDA(ctx, cudaMemcpyAsync(h, hcol + (size_t)re[nread_re].j * ns, sizeof(double) * ns, cudaMemcpyDeviceToHost,
+                                           ctx->stream));
+        }
         MOED_CUDA(ctx, cudaEventRecord(ev[slot], ctx->stream));
         read_j[slot] = j;
-        read_re[slot] = last_re;
-        read_gap[slot] = re.empty() ? 1 : re.back().gap;
         return MO_ED_OK;
     }
 
@@ -888,19 +897,12 @@ struct KryRun {
         seed = seed_;
         base = cycles = m = gn = 0;
         redo = -1;
-        period = f32 ? 6 : 10;
+        ctl = KryPeriod(f32, s.D());
         next_re = 3;
         last_re = -1;
         re.clear();
-        hmax = anorm = 0.0;
-        const double unit = f32 ? 6e-8 : 1.1e-16;
-        const double target = f32 ? 2e-5 : 1e-11, most_h = f32 ? 1e-2 : 1e-4;
-        // The longest period rises while little is found.  In small sectors, where
-        // a reorthogonalisation costs about a step, it does not: one that comes
-        // too late costs a period's steps.  9 million FP32 elements: 79 -> 65 ms.
-        int pmax = f32 ? 16 : 24, ptop = s.D() < (1 << 19) ? pmax : 2 * pmax;
-        int judged = -1, good = -1;   // last reorthogonalisation judged, and found small
-        double grow = 0.0;            // largest growth per step seen
+        nread_re = 0;
+        anorm = 0.0;
         double last_res = 0.0;
         int last_m = 0;
         int j = 0;                    // next step
@@ -926,7 +928,7 @@ struct KryRun {
             const int slot = ndone & 1;
             ++ndone;
             MOED_CUDA(ctx, cudaEventSynchronize(ev[slot]));
-            const double *h = (const double *)ctx->pinned + (size_t)slot * 4 * ns;
+            const double *h = read_at(slot);
             m = read_j[slot];   // alpha[0 .. m), and U_m is the residual vector
             for (int i = 0; i <= m; ++i) {
                 al[i] = h[i];
@@ -938,32 +940,23 @@ struct KryRun {
             const double bd = (f32 ? 1e-5 : 1e-12) * std::max(anorm, 1.0);
             for (int i = base + 1; i <= m; ++i)
                 if (be[i] <= bd) return MO_ED_OK;   // an invariant subspace: thick restarts go on from there
-            if (const int jr = read_re[slot]; jr > 1 && jr != judged) {
+            KryPeriod::Verdict verdict = KryPeriod::kept;
+            for (size_t r = 0; r < read_re[slot].size() && verdict == KryPeriod::kept; ++r) {
+                const KryClean &cl = read_re[slot][r];
                 double c = 0.0;
-                for (int l = 0; l < jr - 1 + (int)front.size(); ++l) c = std::max(c, std::fabs(h[3 * ns + l]));
-                c *= inv[jr];
-                if (!(c < most_h)) {
-                    // orthogonality was lost before this reorthogonalisation:
-                    // back to the last one known to be good, shorter periods
-                    if (good < 0 || read_gap[slot] <= 2) return MO_ED_OK;
-                    ptop = pmax = period = std::max(2, std::min(read_gap[slot], pmax) / 2);
-                    if (int rc = go_back(good)) return rc;
-                    j = good + 1;
-                    full = false;
-                    stop = std::min(j + 4, mmax + 1);
-                    nread = ndone = 0;
-                    last_m = 0;
-                    judged = good;
-                    continue;
-                }
-                judged = good = jr;
-                // Components c taken out once leave c^2 in every vector to come (the
-                // earlier vectors are orthogonal to c only), which does not grow.
-                const int gap = read_gap[slot];
-                grow = std::max(grow, std::max(std::log(c / std::max(2 * unit, hmax * hmax)), 0.3) / gap);
-                hmax = std::max(hmax, c);
-                if (c < target) pmax = std::max(pmax, std::min(ptop, gap + gap / 4 + 1));
-                period = std::max(2, std::min(base > 0 ? std::min(5, pmax) : pmax, (int)(std::log(target / (2 * unit)) / grow)));
+                for (int l = 0; l < cl.j - 1 + (int)front.size(); ++l)
+                    c = std::max(c, std::fabs(h[(3 + r) * ns + l]));
+                verdict = ctl.judge(cl, c * inv[cl.j], base > 0);
+            }
+            if (verdict == KryPeriod::lost) return MO_ED_OK;
+            if (verdict == KryPeriod::back) {
+                if (int rc = go_back(ctl.good)) return rc;
+                j = ctl.good + 1;
+                full = false;
+                stop = std::min(j + 4, mmax + 1);
+                nread = ndone = 0;
+                last_m = 0;
+                continue;
             }
             const double want = tol * std::max(anorm, 1.0);
             double res = 0.0, aim = want;
@@ -1020,7 +1013,6 @@ struct KryRun {
                 j = base + 1;
                 full = false;
                 last_m = 0;
-                judged = good = -1;
                 stop = std::min(base + 12, mmax + 1);
                 nread = ndone = 0;
             }
@@ -1108,8 +1100,8 @@ struct KryRun {
         next_re = base + 1;
         last_re = -1;
         re.clear();
-        hmax = 0.0;
-        period = std::min(period, 4);
+        nread_re = 0;
+        ctl.restart();
         *again = true;
         return MO_ED_OK;
     }
@@ -1120,7 +1112,7 @@ struct KryRun {
     int vectors(int n, std::vector<double> &Y, int ld, int off)
     {
         std::vector<double> Hp;
-        if (hmax > (f32 ? 1e-6 : 1e-12)) {
+        if (ctl.hmax > (f32 ? 1e-6 : 1e-12)) {
             const int nf = (int)front.size();
             std::vector<double> hall((size_t)ns * m);
             MOED_CUDA(ctx, cudaMemcpyAsync(hall.data(), hcol, sizeof(double) * hall.size(), cudaMemcpyDeviceToHost,
@@ -1135,7 +1127,7 @@ struct KryRun {
             // earlier vectors) changes H q_{j-2} and H q'_{j-1}:
             //   column j-2 gains beta_{j-1} g1,
             //   column j-1 gains beta_j g2 + alpha_{j-1} g1 - T g1.
-            for (const Clean &cl : re) {
+            for (const KryClean &cl : re) {
                 const int j = cl.j;
                 if (j >= m) continue;
                 const double *g1 = &hall[(size_t)(j - 1) * ns + nf], *g2 = &hall[(size_t)j * ns + nf];

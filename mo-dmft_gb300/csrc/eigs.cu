@@ -936,8 +936,11 @@ struct KryRun {
                 inv[i] = h[2 * ns + i];
                 if (!std::isfinite(al[i]) || !std::isfinite(be[i]) || !std::isfinite(inv[i])) return MO_ED_OK;
             }
-            for (int i = base; i < m; ++i) anorm = std::max(anorm, std::fabs(al[i]) + be[i + 1]);
-            const double bd = (f32 ? 1e-5 : 1e-12) * std::max(anorm, 1.0);
+            // the norm that tolerances are relative to; scalars of steps that are
+            // about to be discarded can be of any size and must not stay in it
+            double an = anorm;
+            for (int i = base; i < m; ++i) an = std::max(an, std::fabs(al[i]) + be[i + 1]);
+            const double bd = (f32 ? 1e-5 : 1e-12) * std::max(an, 1.0);
             for (int i = base + 1; i <= m; ++i)
                 if (be[i] <= bd) return MO_ED_OK;   // an invariant subspace: thick restarts go on from there
             KryPeriod::Verdict verdict = KryPeriod::kept;
@@ -958,6 +961,7 @@ struct KryRun {
                 last_m = 0;
                 continue;
             }
+            anorm = an;
             const double want = tol * std::max(anorm, 1.0);
             double res = 0.0, aim = want;
             if (!cut) {

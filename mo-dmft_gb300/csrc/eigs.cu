@@ -1118,47 +1118,23 @@ struct KryRun {
         std::vector<double> Hp;
         if (ctl.hmax > (f32 ? 1e-6 : 1e-12)) {
             const int nf = (int)front.size();
-            std::vector<double> hall((size_t)ns * m);
+            std::vector<double> hall((size_t)ns * (m + 1));
             MOED_CUDA(ctx, cudaMemcpyAsync(hall.data(), hcol, sizeof(double) * hall.size(), cudaMemcpyDeviceToHost,
                                            ctx->stream));
             MOED_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-            Hp.assign((size_t)m * m, 0.0);
-            for (int i = 0; i < m; ++i) {
-                Hp[(size_t)i * m + i] = al[i];
-                if (i + 1 < m) Hp[(size_t)i * m + i + 1] = Hp[(size_t)(i + 1) * m + i] = be[i + 1];
-            }
-            // Cleaning q_{j-1} = q'_{j-1} + Q g1 and q_j = q'_j + Q g2 (Q the
-            // earlier vectors) changes H q_{j-2} and H q'_{j-1}:
-            //   column j-2 gains beta_{j-1} g1,
-            //   column j-1 gains beta_j g2 + alpha_{j-1} g1 - T g1.
-            for (const KryClean &cl : re) {
-                const int j = cl.j;
-                if (j >= m) continue;
-                const double *g1 = &hall[(size_t)(j - 1) * ns + nf], *g2 = &hall[(size_t)j * ns + nf];
-                const double s1 = inv[j - 1], s2 = inv[j];
-                double *c2 = j >= 2 ? &Hp[(size_t)(j - 2) * m] : nullptr, *c1 = &Hp[(size_t)(j - 1) * m];
-                for (int l = 0; l < j - 1; ++l) {
-                    if (c2) c2[l] += be[j - 1] * s1 * g1[l];
-                    double tg = al[l] * g1[l];
-                    if (l > 0) tg += be[l] * g1[l - 1];
-                    if (l + 1 < j - 1) tg += be[l + 1] * g1[l + 1];
-                    c1[l] += be[j] * s2 * g2[l] + s1 * (al[j - 1] * g1[l] - tg);
-                }
-                if (j >= 2) c1[j - 1] -= be[j - 1] * s1 * g1[j - 2];
-            }
+            kry_projected(m, al.data(), be.data(), inv.data(), re, hall.data() + nf, ns, Hp);
         }
         // Ritz values that agree to rounding (copies of a degenerate level that
-        // rounding has brought into the run): vectors of T, made orthogonal
-        const double same = 1e-9 * std::max(anorm, 1.0);
+        // rounding has brought into the run): any independent vectors of them
+        const double same = (f32 ? 1e-6 : 1e-9) * std::max(anorm, 1.0);
         std::vector<const double *> prev;
         for (int i = 0; i < n; ++i) {
             double *yi = &Y[(size_t)i * ld + off];
             if (i > 0 && th[i] - th[i - 1] > same) prev.clear();
-            const bool cluster = !prev.empty() || (i + 1 < n && th[i + 1] - th[i] <= same);
-            if (Hp.empty() || cluster)
+            if (Hp.empty())
                 tri_eigvec(m, al.data(), be.data() + 1, th[i], yi, prev.data(), (int)prev.size());
             else
-                hess_eigvec(m, Hp.data(), m, th[i], anorm, yi);
+                hess_eigvec(m, Hp.data(), m, th[i], anorm, yi, prev.data(), (int)prev.size());
             prev.push_back(yi);
         }
         for (int i = 0; i < n; ++i)
@@ -1205,6 +1181,7 @@ int plz_solve(mo_ed_ctx *ctx, const Sector &s, int nev, std::vector<double> &val
                            vecs || search ? &X : nullptr);
     if (rc == MO_ED_ERR_NOCONV || rc == MO_ED_ERR_NOMEM) return MO_ED_OK;   // the thick restarts try
     if (rc) return rc;
+    if (!(ctx->diag_res_true <= kry_residual_limit(f32, tol, run.anorm))) return MO_ED_OK;
     // A Krylov space holds one vector of each eigenspace.  Where the model can
     // have exactly degenerate levels, runs orthogonal to the states found look
     // for others below the highest of them, until one finds none.

@@ -237,8 +237,10 @@ inline void tri_eigvec(int n, const double *d, const double *e, double theta, do
 // leading dimension ld) for its eigenvalue theta: two steps of inverse
 // iteration with the LU factors of h - theta I (partial pivoting between
 // neighbouring rows, the only ones that can hold the pivot).  scale: a norm
-// of h; a pivot below 2^-52 scale is replaced by that.
-inline void hess_eigvec(int n, const double *h, int ld, double theta, double scale, double *y)
+// of h; a pivot below 2^-52 scale is replaced by that.  prev[0 .. nprev): unit
+// vectors of (nearly) the same eigenvalue that y has to be orthogonal to.
+inline void hess_eigvec(int n, const double *h, int ld, double theta, double scale, double *y,
+                        const double *const *prev = nullptr, int nprev = 0)
 {
     const double tiny = 2.220446049250313e-16 * scale;
     std::vector<double> u((size_t)n * n, 0.0), l(n, 0.0);   // u row-major
@@ -257,8 +259,8 @@ inline void hess_eigvec(int n, const double *h, int ld, double theta, double sca
         for (int j = k + 1; j < n; ++j) U(k + 1, j) -= l[k] * U(k, j);
     }
     if (std::fabs(U(n - 1, n - 1)) < tiny) U(n - 1, n - 1) = tiny;
-    for (int i = 0; i < n; ++i) y[i] = 1.0 + 0.37 * (i % 7);   // no structure in common with an eigenvector
-    for (int it = 0; it < 2; ++it) {
+    for (int i = 0; i < n; ++i) y[i] = 1.0 + 0.37 * ((i + 3 * nprev * (i % 5)) % 7);   // no structure in common with an eigenvector
+    for (int it = 0; it < (nprev ? 3 : 2); ++it) {
         for (int k = 0; k + 1 < n; ++k) {
             if (swp[k]) std::swap(y[k], y[k + 1]);
             y[k + 1] -= l[k] * y[k];
@@ -271,10 +273,14 @@ inline void hess_eigvec(int n, const double *h, int ld, double theta, double sca
         double s = 0.0;
         for (int i = 0; i < n; ++i) s = std::max(s, std::fabs(y[i]));
         double q = 0.0;
-        for (int i = 0; i < n; ++i) {
-            y[i] /= s;
-            q += y[i] * y[i];
-        }
+        for (int i = 0; i < n; ++i) y[i] /= s;
+        for (int pass = 0; pass < 2; ++pass)
+            for (int k = 0; k < nprev; ++k) {
+                double c = 0.0;
+                for (int i = 0; i < n; ++i) c += y[i] * prev[k][i];
+                for (int i = 0; i < n; ++i) y[i] -= c * prev[k][i];
+            }
+        for (int i = 0; i < n; ++i) q += y[i] * y[i];
         q = 1.0 / std::sqrt(q);
         for (int i = 0; i < n; ++i) y[i] *= q;
     }

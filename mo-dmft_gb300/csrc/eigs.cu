@@ -75,13 +75,14 @@ struct KryScal {
     double *alpha, *beta, *inv;
 };
 
-// the scalars of step j from ||U_j||^2 and U_j . H U_j
+// the scalars of step j from ||U_j||^2 and U_j . H U_j (zeros where the Krylov
+// space has closed: the vectors to come are zero then)
 __device__ __forceinline__ void kry_store(const KryScal &sc, int j, double n2, double d)
 {
-    const double inv = rsqrt_pos(n2);
+    const double inv = n2 > 0.0 ? rsqrt_pos(n2) : 0.0;
     sc.inv[j] = inv;
     sc.beta[j] = n2 * inv;
-    sc.alpha[j] = d * rcp_pos(n2);
+    sc.alpha[j] = n2 > 0.0 ? d * rcp_pos(n2) : 0.0;
 }
 
 // the same from the partials of step j
@@ -297,7 +298,8 @@ k_kry_cluster(const __grid_constant__ HvJobT<T> jb, const ModelDev *__restrict__
             for (int o = 8; o > 1; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
             const double d = __shfl_sync(0xffffffffu, v, 1), n2 = given ? s_n0 : v;
             if (lane == 0) {
-                const double in = rsqrt_pos(n2), be = n2 * in, al = d * rcp_pos(n2);
+                double al, be, in;
+                kry_store(KryScal{&al, &be, &in}, 0, n2, d);
                 if (rank == 0) {
                     sc.alpha[j] = al;
                     sc.beta[j] = be;
@@ -889,8 +891,14 @@ struct KryRun {
 
     // The run from a random vector.  cut null: until the nwant lowest Ritz
     // pairs have converged.  cut: until every Ritz value below *cut has
-    // converged and the next one is known to a tenth of its distance from the
+    // converged and the next one is known to kSettled of its distance from the
     // cut (*nlow = how many lie below).  *ok = false: gave up.
+    //
+    // A Ritz value above the cut can stand still for a while before it falls to
+    // a level below that the start vector has a small share of.  Its residual
+    // then is that share's angle times the distance, so kSettled bounds the
+    // angle; random shares a tenth of their neighbours' are common.
+    static constexpr double kSettled = 1e-3;
     int go(unsigned long long seed_, const double *cut, int *nlow, bool *ok)
     {
         *ok = false;
@@ -939,13 +947,20 @@ struct KryRun {
             // the norm that tolerances are relative to; scalars of steps that are
             // about to be discarded can be of any size and must not stay in it
             double an = anorm;
-            for (int i = base; i < m; ++i) an = std::max(an, std::fabs(al[i]) + be[i + 1]);
-            const double bd = (f32 ? 1e-5 : 1e-12) * std::max(an, 1.0);
-            for (int i = base + 1; i <= m; ++i)
-                if (be[i] <= bd) return MO_ED_OK;   // an invariant subspace: thick restarts go on from there
+            bool closed = false;   // the Krylov space ends at U_{m-1}
+            for (int i = base; i < m && !closed; ++i) {
+                an = std::max(an, std::fabs(al[i]) + be[i + 1]);
+                if (be[i + 1] > (f32 ? 1e-5 : 1e-12) * std::max(an, 1.0)) continue;
+                if (!cut) return MO_ED_OK;   // an invariant subspace: thick restarts go on from there
+                // it has a vector of every eigenspace but the found states': the
+                // search ends here
+                m = i + 1;
+                closed = true;
+            }
             KryPeriod::Verdict verdict = KryPeriod::kept;
             for (size_t r = 0; r < read_re[slot].size() && verdict == KryPeriod::kept; ++r) {
                 const KryClean &cl = read_re[slot][r];
+                if (cl.j >= m + !closed) break;
                 double c = 0.0;
                 for (int l = 0; l < cl.j - 1 + (int)front.size(); ++l)
                     c = std::max(c, std::fabs(h[(3 + r) * ns + l]));
@@ -989,14 +1004,14 @@ struct KryRun {
                 bool settled = res <= want;
                 if (n < k) {   // the first value above the cut
                     tri_eigvec(m, al.data(), be.data() + 1, th[n], y.data());
-                    const double r = std::fabs(be[m] * y[m - 1]), lim = std::max(0.1 * (th[n] - *cut), want);
+                    const double r = std::fabs(be[m] * y[m - 1]), lim = std::max(kSettled * (th[n] - *cut), want);
                     if (r > lim) settled = false;
                     if (n == 0) {
                         res = r;
                         aim = lim;
                     }
                 }
-                if (settled || full) {
+                if (settled || closed) {
                     *ok = settled;
                     return MO_ED_OK;
                 }
@@ -1010,7 +1025,8 @@ struct KryRun {
             if (!full) {
                 stop = std::min(std::max(j + 4, m + std::min(ahead, 40)), mmax + 1);
             } else if (ndone == nread) {
-                if (++cycles >= ctx->opt.gs_maxcycles) return fail(ctx, MO_ED_ERR_NOCONV, "eigensolver did not converge");
+                if (++cycles >= ctx->opt.gs_maxcycles)
+                    return cut ? (int)MO_ED_OK : fail(ctx, MO_ED_ERR_NOCONV, "eigensolver did not converge");
                 bool again = false;
                 if (int rc = restart(&again)) return rc == MO_ED_ERR_NOMEM ? (int)MO_ED_OK : rc;
                 if (!again) return MO_ED_OK;
@@ -1175,26 +1191,37 @@ int plz_solve(mo_ed_ctx *ctx, const Sector &s, int nev, std::vector<double> &val
     if (int rc = run.vectors(nev, Y, run.m, 0)) return rc;
     MOED_CUDA(ctx, cudaMemcpyAsync(run.hcol, Y.data(), sizeof(double) * Y.size(), cudaMemcpyHostToDevice, ctx->stream));
     std::vector<DevBuf> X;
-    const bool search = ctx->degenerate;
     const int cycles = run.cycles;
     int rc = ritz_pairs<T>(ctx, s, run.basis(run.m), run.m, run.hcol, nev, nev, run.matvecs, vals,
-                           vecs || search ? &X : nullptr);
+                           vecs || ctx->degenerate ? &X : nullptr);
     if (rc == MO_ED_ERR_NOCONV || rc == MO_ED_ERR_NOMEM) return MO_ED_OK;   // the thick restarts try
     if (rc) return rc;
     if (!(ctx->diag_res_true <= kry_residual_limit(f32, tol, run.anorm))) return MO_ED_OK;
     // A Krylov space holds one vector of each eigenspace.  Where the model can
     // have exactly degenerate levels, runs orthogonal to the states found look
-    // for others below the highest of them, until one finds none.
-    for (int round = 1; search && round <= 2 * nev + 2; ++round) {
+    // for others below the highest of them, until one finds none.  A run that
+    // gives up says nothing: others from other vectors take its place, and after
+    // three of them the thick restarts do.
+    const double norm = std::max(run.anorm, 1.0);
+    bool complete = !ctx->degenerate;
+    for (int round = 1, lost = 0; !complete && lost < 3 && round <= 2 * nev + 5; ++round) {
         run.front.clear();
         for (const DevBuf &b : X) run.front.push_back((const T *)b.p);
-        const double cut = vals[nev - 1] - 10 * tol * std::max(run.anorm, 1.0);
+        const double cut = vals[nev - 1] - 10 * tol * norm;
         int nlow = 0;
         run.matvecs = 0;
         if (int r2 = run.go(seed + 7919ULL * round, &cut, &nlow, &ok)) return r2;
         const long long mv = ctx->diag_matvecs + run.matvecs;
+        const double res = ctx->diag_res_true;
         ctx->diag_matvecs = mv;
-        if (!ok || nlow == 0) break;
+        if (!ok) {
+            ++lost;
+            continue;
+        }
+        if (nlow == 0) {
+            complete = true;
+            break;
+        }
         const int n = nev + nlow, mm = nev + run.m;
         Y.assign((size_t)mm * n, 0.0);
         for (int i = 0; i < nev; ++i) Y[(size_t)i * mm + i] = 1.0;
@@ -1205,12 +1232,18 @@ int plz_solve(mo_ed_ctx *ctx, const Sector &s, int nev, std::vector<double> &val
         std::vector<double> v2;
         std::vector<DevBuf> X2;
         rc = ritz_pairs<T>(ctx, s, run.basis(run.m), mm, run.hcol, n, n, mv, v2, &X2);
-        if (rc == MO_ED_ERR_NOCONV || rc == MO_ED_ERR_NOMEM) break;
-        if (rc) return rc;
+        if (rc == MO_ED_ERR_NOMEM) break;
+        if (rc && rc != MO_ED_ERR_NOCONV) return rc;
+        if (rc || !(ctx->diag_res_true <= kry_residual_limit(f32, tol, norm))) {
+            ++lost;
+            ctx->diag_res_true = res;
+            continue;
+        }
         X2.resize(nev);
         X = std::move(X2);
         vals.assign(v2.begin(), v2.begin() + nev);
     }
+    if (!complete) return MO_ED_OK;
     ctx->diag_cycles = cycles + 1;
     if (vecs) *vecs = std::move(X);
     *done = true;

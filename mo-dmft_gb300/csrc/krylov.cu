@@ -744,6 +744,12 @@ static int trl_solve(mo_ed_ctx *ctx, const Sector &s, int nev, std::vector<doubl
     bool done = false;
     int cycle = 0;
     double anorm = 0.0;
+    // A Krylov space holds one vector of each eigenspace.  Where the model can
+    // have exactly degenerate levels, the converged vectors are
+    // kept and a fresh random direction goes on from there, until one adds no
+    // level to the lowest ones: the values before it, or empty
+    std::vector<double> known;
+    const bool search = ctx->degenerate && ncv >= nwant + 2;
     for (; cycle < ctx->opt.gs_maxcycles && !done; ++cycle) {
         m = ncv;
         // The steps of a cycle run without a host round trip; the diagonal and
@@ -823,13 +829,37 @@ static int trl_solve(mo_ed_ctx *ctx, const Sector &s, int nev, std::vector<doubl
         const size_t h = res_hist.size();
         const bool stalled = prec == MO_ED_FP32 && h >= 6 && maxres <= 1e-6 * std::max(anorm, 1.0) &&
                              maxres > 0.9 * res_hist[h - 6];
-        if (nconv >= nwant || m >= D || stalled) {
+        const bool converged = nconv >= nwant || stalled;
+        if (m >= D || (converged && (!search || cycle + 1 >= ctx->opt.gs_maxcycles))) {
             done = true;
             break;
         }
         // thick restart: keep kkeep lowest Ritz vectors, then the residual vector
         // after a breakdown every Ritz vector of the invariant subspace is kept
-        const int kk = broke ? std::min(kkeep, m) : std::min(kkeep, m - 1);
+        bool fresh = broke;
+        int kk = broke ? std::min(kkeep, m) : std::min(kkeep, m - 1);
+        if (converged) {
+            // the value after the wanted ones has to be known as well (1e-3 of
+            // its distance from them: KryRun::go, eigs.cu; 1e-6 is where FP32
+            // residuals stop falling)
+            const double an = std::max(anorm, 1.0);
+            bool settled = known.empty() || broke;
+            if (!settled && m > nwant)
+                settled = std::fabs(beta_m * evecs_h[(size_t)nwant * m + (m - 1)]) <=
+                          std::max(1e-3 * (theta[nwant] - theta[nwant - 1]), (prec == MO_ED_FP32 ? 1e-6 : tol) * an);
+            if (settled) {
+                bool same = !known.empty();
+                for (size_t i = 0; i < known.size(); ++i) same = same && known[i] - theta[i] <= 10 * tol * an;
+                if (same) {
+                    done = true;
+                    break;
+                }
+                known.assign(theta.begin(), theta.begin() + nwant);
+                res_hist.clear();
+                fresh = true;
+                kk = nwant;   // converged vectors only: the others leave a residual along V_m
+            }
+        }
         VPtrs<T> P = make_ptrs<T>(V, m);
         for (int c0 = 0; c0 < kk; c0 += 8) {
             const int nc = std::min(8, kk - c0);
@@ -838,8 +868,8 @@ static int trl_solve(mo_ed_ctx *ctx, const Sector &s, int nev, std::vector<doubl
             if (int rc = rotate<T>(ctx, G, P, m, (const double *)devecs.p, m, c0, nc, X, Dp)) return rc;
         }
         for (int i = 0; i < kk; ++i) std::swap(V[i], spare[i]);
-        if (broke) {
-            // invariant subspace: continue from a fresh random direction
+        if (fresh) {
+            // invariant subspace, or a search: continue from a fresh random direction
             k_random<T><<<G, kVecThreads, 0, ctx->stream>>>((T *)W->p, Dp, s.ld(), s.up->n,
                                                             seed + 7919ULL * (cycle + 1) * kTrlMaxNcv);
             MOED_CHECK_LAUNCH(ctx);

@@ -40,3 +40,20 @@ def test_equal_baths(solver, oracle, precision, sym, norb, nbath, secs):
     for nu, nd in secs:
         w = dense(oracle, norb, nbath, U, J, ek, vk, nu, nd)
         check(solver, precision, norb, nbath, U, J, ek, vk, nu, nd, w, (3, 4, 6, 12, 20))
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_thick_restarts(solver, oracle, precision):
+    """Sectors of 90 to 225 states, below the line of the unrestarted solver, and
+    a given Krylov dimension."""
+    norb, nbath, U, J = 3, 3, 3.0, 0.5
+    rng = np.random.default_rng(1)
+    ek = np.concatenate([levels(norb, U, J), np.full(3, rng.uniform(-1, 1))])
+    vk = np.eye(3) * rng.uniform(0.1, 0.5)
+    try:
+        for nu, nd, nevs, ncv in ((1, 3, (3, 6, 12), 0), (2, 1, (3, 6, 12), 0), (2, 2, (20,), 0), (3, 3, (3, 6, 12), 30)):
+            w = dense(oracle, norb, nbath, U, J, ek, vk, nu, nd)
+            solver.set_options(gs_ncv=ncv)
+            check(solver, precision, norb, nbath, U, J, ek, vk, nu, nd, w, nevs)
+    finally:
+        solver.set_options(gs_ncv=0)

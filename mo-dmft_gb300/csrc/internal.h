@@ -261,7 +261,7 @@ struct mo_ed_ctx {
     std::vector<int> cpl_orb, cpl_bath;  // nonzero couplings in reference loop order
     std::vector<double> cpl_val;
     std::vector<int> site_subsys;  // conserved subsystem (orbital + coupled bath levels) of each site
-    // the model can have exactly degenerate levels within a sector
+    // the model can have exactly degenerate levels within a sector (degeneracy.h)
     bool degenerate = false;
     int dblk_bound = 0;            // largest down-spin block over every electron count
     int dblk_mv_bound = 0;         // most hybridisation moves in one such block

@@ -10,9 +10,9 @@
 // (combinatorial number system) and a rank is unranked greedily from the top
 // bit.  Both directions are one thread per element here.
 #include <algorithm>
-#include <cmath>
 #include <cstring>
 
+#include "degeneracy.h"
 #include "internal.h"
 
 namespace moed {
@@ -368,30 +368,7 @@ int build_model(mo_ed_ctx *ctx)
             ctx->dblk_mv_bound = (int)std::max<long long>(ctx->dblk_mv_bound, kv.second.second);
         }
     }
-    // Levels of a sector can be degenerate by symmetry only where the model has
-    // a symmetry beyond the spin rotation (whose multiplets have one member per
-    // sector): a rotation among orbitals or bath levels needs two bath levels
-    // of one energy, two uncoupled orbitals, or a bath level coupled to
-    // nothing; without J each orbital's spin rotates by itself.  Near-equal
-    // energies count: they split levels by less than a Lanczos run resolves.
-    {
-        bool deg = norb > 1 && std::fabs(ctx->J) < 1e-3;
-        int free_orb = 0;
-        for (int io = 0; io < norb; ++io) {
-            bool coupled = false;
-            for (int ib = 0; ib < nbath; ++ib) coupled |= ctx->vk[(size_t)ib * norb + io] != 0.0;
-            free_orb += !coupled;
-        }
-        deg |= free_orb > 1;
-        for (int ib = 0; ib < nbath; ++ib) {
-            bool coupled = false;
-            for (int io = 0; io < norb; ++io) coupled |= std::fabs(ctx->vk[(size_t)ib * norb + io]) > 1e-3;
-            deg |= !coupled;
-            for (int jb = 0; jb < ib; ++jb)
-                deg |= std::fabs(ctx->ek[norb + ib] - ctx->ek[norb + jb]) <= 1e-3 * std::max(1.0, std::fabs(ctx->ek[norb + ib]));
-        }
-        ctx->degenerate = deg;
-    }
+    ctx->degenerate = can_be_degenerate(norb, nbath, ctx->U, ctx->J, ctx->ek.data() + norb, ctx->vk.data());
     if (!ctx->d_mdl) MOED_CUDA(ctx, cudaMalloc(&ctx->d_mdl, sizeof(ModelDev)));
     MOED_CUDA(ctx, cudaMemcpyAsync(ctx->d_mdl, &m, sizeof(m), cudaMemcpyHostToDevice, ctx->stream));
     MOED_CUDA(ctx, cudaStreamSynchronize(ctx->stream));

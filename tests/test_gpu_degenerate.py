@@ -1,7 +1,12 @@
 """Eigensolves of models with exactly degenerate levels, where a single Krylov
-space holds one member of each level.  The lowest levels with their
-multiplicities against dense diagonalisation of the oracle's H.  Bounds: those of the other
+space holds one member of each level: equal baths, spins that rotate
+separately (U = 0), orbitals that couple alike or in fewer combinations than
+there are orbitals, baths that are each other's mirror image.
+The lowest levels with their multiplicities against sums of one-spin levels
+(U = 0) or dense diagonalisation of the oracle's H.  Bounds: those of the other
 eigensolver tests (1e-9 FP64, 1e-8 FP32)."""
+import itertools
+
 import numpy as np
 import pytest
 
@@ -57,3 +62,45 @@ def test_thick_restarts(solver, oracle, precision):
             check(solver, precision, norb, nbath, U, J, ek, vk, nu, nd, w, nevs)
     finally:
         solver.set_options(gs_ncv=0)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("seed", range(4))
+def test_free_spins(solver, precision, seed):
+    rng = np.random.default_rng(seed)
+    nbath, nu, nd = 7, 4, 4
+    ek = np.concatenate([[rng.uniform(-0.5, 0.5)], rng.uniform(-1, 1, nbath)])
+    vk = rng.uniform(0.1, 0.6, (1, nbath))
+    h = np.diag(ek)
+    h[0, 1:] = h[1:, 0] = vk[0]
+    one = np.array([sum(c) for c in itertools.combinations(np.linalg.eigvalsh(h), nu)])
+    w = np.sort((one[:, None] + one[None, :]).ravel())
+    check(solver, precision, 1, nbath, 0.0, 0.0, ek, vk, nu, nd, w, (3, 4, 8))
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("seed", range(200, 203))
+def test_dependent_couplings(solver, oracle, precision, seed):
+    rng = np.random.default_rng(seed)
+    U, J = 3.0, 0.5
+    for norb, nbath in ((3, 3), (3, 4), (4, 2), (4, 3)):
+        vk = np.tile(rng.uniform(0.1, 0.5, nbath), (3, 1)) if norb == 3 else \
+            rng.uniform(-1, 1, (norb, 2)) @ rng.uniform(0.1, 0.5, (2, nbath))
+        ek = np.concatenate([levels(norb, U, J), rng.uniform(-1, 1, nbath)])
+        n = norb + nbath
+        for nu, nd in ((n // 2, n // 2), (n // 2 - 1, n // 2)):
+            w = dense(oracle, norb, nbath, U, J, ek, vk, nu, nd)
+            check(solver, precision, norb, nbath, U, J, ek, vk, nu, nd, w, (3, 4, 6, 12, 20))
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("seed", range(3))
+def test_mirrored_baths(solver, oracle, precision, seed):
+    rng = np.random.default_rng(seed)
+    e, v = rng.uniform(-1, 1, 2), rng.uniform(0.1, 0.5, 2)
+    U, J = 4.0, 1.0
+    ek = np.concatenate([levels(2, U, J), e, -e])
+    vk = np.kron(np.eye(2), v[None, :])
+    for nu, nd in ((3, 3), (2, 4)):
+        w = dense(oracle, 2, 4, U, J, ek, vk, nu, nd)
+        check(solver, precision, 2, 4, U, J, ek, vk, nu, nd, w, (3, 4, 6, 12))

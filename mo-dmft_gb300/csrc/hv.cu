@@ -1431,7 +1431,7 @@ k_hv_wide(const __grid_constant__ HvBatch<float> batch, const ModelDev *__restri
         }
         __syncthreads();
         const bool want_dot = jb.dot_partial != nullptr;
-        float part = 0.f;
+        double dacc = 0.0;
         const int nunit = (ld + 63) >> 6;
         for (int c = warp; c < nunit; c += NW) {
             const int u = 64 * c + 2 * lane;
@@ -1549,6 +1549,8 @@ k_hv_wide(const __grid_constant__ HvBatch<float> batch, const ModelDev *__restri
                     if (d >= 0) *reinterpret_cast<float2 *>(y + (size_t)d * ld + u) = make_float2(acc[0][r], acc[1][r]);
                 }
                 if (want_dot) {   // rows that are not there are staged as zeros
+                    // 2 R products in FP32, then FP64, as k_hv_async
+                    float part = 0.f;
 #pragma unroll
                     for (int k = 0; k < 2; ++k)
 #pragma unroll
@@ -1557,11 +1559,11 @@ k_hv_wide(const __grid_constant__ HvBatch<float> batch, const ModelDev *__restri
                             const float *a = acc[k] + 4 * p;
                             part += (xa.x * a[0] + xa.y * a[1]) + (xa.z * a[2] + xa.w * a[3]);
                         }
+                    dacc += widen(part);
                 }
             }
         }
         if (want_dot) {
-            double dacc = (double)part;
             for (int off = 16; off > 0; off >>= 1) dacc += __shfl_down_sync(0xffffffffu, dacc, off);
             if (lane == 0) s_red[warp] = dacc;
             __syncthreads();

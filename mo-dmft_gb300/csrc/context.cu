@@ -10,8 +10,13 @@ namespace moed {
 void DevBuf::release()
 {
     if (slab) slab.reset();
+    else if (p && pooled) {
+        cudaFreeAsync(p, stream);
+        cudaStreamSynchronize(stream);   // only then can others have it
+    }
     else if (p) cudaFree(p);
     p = nullptr;
+    pooled = false;
     bytes = 0;
 }
 
@@ -32,9 +37,11 @@ int dev_alloc(mo_ed_ctx *ctx, DevBuf &b, size_t bytes)
     b.release();
     if (bytes == 0) bytes = 16;
     cudaError_t e = cudaMalloc(&b.p, bytes);
-    if (e == cudaErrorMemoryAllocation && !ctx->kry_busy && !ctx->kry_pool.empty()) {
+    if (e == cudaErrorMemoryAllocation && ctx->mem_pool) {
+        // frees of the pool may still be on their way
         cudaGetLastError();
-        ctx->kry_pool.clear();   // the Krylov vectors kept between solves
+        cudaStreamSynchronize(ctx->stream);
+        cudaMemPoolTrimTo(ctx->mem_pool, 0);
         e = cudaMalloc(&b.p, bytes);
     }
     if (e != cudaSuccess) {
@@ -43,6 +50,31 @@ int dev_alloc(mo_ed_ctx *ctx, DevBuf &b, size_t bytes)
         return cuda_fail(ctx, e, "cudaMalloc");
     }
     b.bytes = bytes;
+    return MO_ED_OK;
+}
+
+int pool_alloc(mo_ed_ctx *ctx, DevBuf &b, size_t bytes)
+{
+    b.release();
+    if (!ctx->mem_pool) {
+        cudaMemPoolProps props = {};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = ctx->device;
+        MOED_CUDA(ctx, cudaMemPoolCreate(&ctx->mem_pool, &props));
+        unsigned long long keep = (ctx->worker ? 4ull : 24ull) << 30;
+        MOED_CUDA(ctx, cudaMemPoolSetAttribute(ctx->mem_pool, cudaMemPoolAttrReleaseThreshold, &keep));
+    }
+    if (bytes == 0) bytes = 16;
+    const cudaError_t e = cudaMallocFromPoolAsync(&b.p, bytes, ctx->mem_pool, ctx->stream);
+    if (e != cudaSuccess) {
+        b.p = nullptr;
+        cudaGetLastError();
+        return cuda_fail(ctx, e, "cudaMallocFromPoolAsync");
+    }
+    b.bytes = bytes;
+    b.pooled = true;
+    b.stream = ctx->stream;
     return MO_ED_OK;
 }
 
@@ -187,6 +219,7 @@ int mo_ed_destroy(mo_ed_ctx *ctx)
     ctx->states.clear();
     if (ctx->d_mdl) cudaFree(ctx->d_mdl);
     if (ctx->pinned) cudaFreeHost(ctx->pinned);
+    if (ctx->mem_pool) cudaMemPoolDestroy(ctx->mem_pool);
     if (ctx->own_stream) cudaStreamDestroy(ctx->stream);
     delete ctx;
     return MO_ED_OK;

@@ -52,11 +52,7 @@ namespace cg = cooperative_groups;
 constexpr int kKryMax = 488, kKryWide = 117;           // more vectors than kKryWide to start with: thick restarts
 constexpr size_t kKryRunBytes = (size_t)128 << 30;
 constexpr long long kKryMinDim = 128;                  // smaller sectors: thick restarts (krylov.cu)
-// Krylov vectors kept in the context between solves: up to the first without
-// asking; up to the second (not in the worker contexts of a solve) while that is
-// at most a quarter of the free memory.  20 GB of an eigensolve of 15 million
-// FP32 elements: 10 ms to allocate in 240 MB chunks and 17 ms to free, of 150.
-constexpr size_t kKryPoolBytes = (size_t)4 << 30, kKryKeepBytes = (size_t)24 << 30;
+constexpr size_t kKryAskBytes = (size_t)4 << 30;       // runs that may need more look at the free memory first
 constexpr size_t kRrPoolBytes = (size_t)64 << 20;      // largest FP64 vector of the pooled Rayleigh-Ritz workspace
 constexpr size_t kSlabBytes = (size_t)1 << 20;         // returned vectors up to this size share one allocation
 // k_kry_cluster: sectors up to these sizes, shared memory of a CTA.  4 states
@@ -557,46 +553,40 @@ template int ritz_pairs<double>(mo_ed_ctx *, const Sector &, const VPtrs<double>
 // ---------------------------------------------------------------------------
 namespace {
 
-// Krylov vectors in chunks, allocated as the run reaches them
+// Krylov vectors in chunks, allocated as the run reaches them: the first kHold
+// bytes stay with the context (the sectors of a solve of many small ones), the
+// others come from its pool
 struct KryVectors {
+    static constexpr size_t kHold = (size_t)64 << 20;
     mo_ed_ctx *ctx;
-    size_t vb;
+    size_t vb, held = 0;
     int per;                             // vectors per chunk
-    std::vector<DevBuf> local;           // chunks past those of the context's pool
+    size_t nheld = 0;
+    std::vector<DevBuf> chunks;
     std::vector<void *> p;               // vector j
-    size_t chunks = 0;
-    bool pooled = true;
     KryVectors(mo_ed_ctx *c, size_t bytes) : ctx(c), vb((bytes + 255) & ~(size_t)255)
     {
         per = (int)std::max<size_t>(1, std::min<size_t>(32, ((size_t)1 << 30) / vb));
-        ctx->kry_busy = true;
     }
-    ~KryVectors() { ctx->kry_busy = false; }
     KryVectors(const KryVectors &) = delete;
-    // whether the pool may hold `bytes` in chunk i
-    bool keeps(size_t i, size_t bytes) const
-    {
-        size_t total = bytes;
-        for (size_t k = 0; k < ctx->kry_pool.size(); ++k)
-            if (k != i) total += ctx->kry_pool[k].bytes;
-        if (total <= kKryPoolBytes) return true;
-        if (ctx->worker || total > kKryKeepBytes) return false;
-        size_t fr = 0, tot = 0;
-        return cudaMemGetInfo(&fr, &tot) == cudaSuccess && total <= fr / 4;
-    }
     int grow(int n)                      // vectors 0 .. n-1 exist
     {
         while ((int)p.size() < n) {
             const size_t need = vb * (size_t)per;
-            if (pooled) {
-                if (ctx->kry_pool.size() <= chunks) ctx->kry_pool.resize(chunks + 1);
-                pooled = ctx->kry_pool[chunks].bytes >= need || keeps(chunks, need);
+            void *base;
+            if (held + need <= kHold) {
+                std::vector<DevBuf> &h = ctx->kry_hold;
+                if (h.size() <= nheld) h.resize(nheld + 1);
+                if (int rc = ensure(ctx, h[nheld], need)) return rc;
+                base = h[nheld++].p;
+                held += need;
+            } else {
+                DevBuf b;
+                if (int rc = pool_alloc(ctx, b, need)) return rc;
+                base = b.p;
+                chunks.push_back(std::move(b));
             }
-            if (!pooled) local.emplace_back();
-            DevBuf &b = pooled ? ctx->kry_pool[chunks] : local.back();
-            if (int rc = ensure(ctx, b, need)) return rc;
-            for (int i = 0; i < per; ++i) p.push_back((char *)b.p + vb * i);
-            ++chunks;
+            for (int i = 0; i < per; ++i) p.push_back((char *)base + vb * i);
         }
         return MO_ED_OK;
     }
@@ -1174,10 +1164,15 @@ int plz_solve(mo_ed_ctx *ctx, const Sector &s, int nev, std::vector<double> &val
     const size_t vb = sizeof(T) * (size_t)s.Dpad();
     // room for the front vectors of the search below: nev
     int mmax = (int)std::min<long long>(kKryMax - nev, 3 * D / 4);
-    if (vb * (size_t)mmax > kKryPoolBytes) {
+    if (vb * (size_t)mmax > kKryAskBytes) {
         size_t fr = 0, tot = 0;
         MOED_CUDA(ctx, cudaMemGetInfo(&fr, &tot));
-        for (const DevBuf &b : ctx->kry_pool) fr += b.bytes;
+        if (ctx->mem_pool) {   // what idles in the pool is free
+            unsigned long long held = 0, used = 0;
+            MOED_CUDA(ctx, cudaMemPoolGetAttribute(ctx->mem_pool, cudaMemPoolAttrReservedMemCurrent, &held));
+            MOED_CUDA(ctx, cudaMemPoolGetAttribute(ctx->mem_pool, cudaMemPoolAttrUsedMemCurrent, &used));
+            fr += (size_t)(held - used);
+        }
         mmax = (int)std::min<size_t>(mmax, std::min(kKryRunBytes, fr / 2) / vb);
         if (mmax < least + 40) return MO_ED_OK;
     }

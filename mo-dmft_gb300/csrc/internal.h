@@ -194,16 +194,18 @@ struct HvJobT {
 // ---------------------------------------------------------------------------
 // context
 // ---------------------------------------------------------------------------
-constexpr size_t kLzPoolBytes = (size_t)512 << 20;
+constexpr size_t kLzHoldBytes = (size_t)64 << 20;
 
 struct DevBuf {              // owning device allocation (move-only)
     void *p = nullptr;
     size_t bytes = 0;
     std::shared_ptr<void> slab;   // set: p is a part of this allocation, shared with others
+    bool pooled = false;          // pool_alloc: freed in the order of this stream
+    cudaStream_t stream = nullptr;
     DevBuf() = default;
     DevBuf(const DevBuf &) = delete;
     DevBuf &operator=(const DevBuf &) = delete;
-    DevBuf(DevBuf &&o) noexcept : p(o.p), bytes(o.bytes), slab(std::move(o.slab))
+    DevBuf(DevBuf &&o) noexcept : p(o.p), bytes(o.bytes), slab(std::move(o.slab)), pooled(o.pooled), stream(o.stream)
     {
         o.p = nullptr;
         o.bytes = 0;
@@ -215,6 +217,8 @@ struct DevBuf {              // owning device allocation (move-only)
             p = o.p;
             bytes = o.bytes;
             slab = std::move(o.slab);
+            pooled = o.pooled;
+            stream = o.stream;
             o.p = nullptr;
             o.bytes = 0;
         }
@@ -294,15 +298,15 @@ struct mo_ed_ctx {
     // eigensolver workspace reused across sectors (Krylov vectors of sectors
     // up to 64 MB per vector, and the projected-problem arrays)
     std::vector<moed::DevBuf> trl_pool, trl_small, rr_pool;
-    // eigs.cu: chunks of Krylov vectors kept between solves (KryVectors; given
-    // back when an allocation fails while no run uses them), small arrays, and pinned host memory for the
-    // coefficients read while the next steps run
-    std::vector<moed::DevBuf> kry_pool, kry_small;
-    bool kry_busy = false, worker = false;
+    // eigs.cu: small arrays, and pinned host memory for the coefficients read
+    // while the next steps run
+    std::vector<moed::DevBuf> kry_small, kry_hold;
+    moed::DevBuf lz_hold;      // workspace of lanczos_iteration and the Green's function, up to kLzHoldBytes
+    bool worker = false;       // a context of solve_sectors' threads
+    cudaMemPool_t mem_pool = nullptr;   // pool_alloc
     // where the next small returned vectors go (dev_alloc_slab)
     std::shared_ptr<void> slab;
     size_t slab_used = 0;
-    moed::DevBuf lz_pool;      // workspace of lanczos_iteration and the Green's function, up to kLzPoolBytes
     void *pinned = nullptr;
     size_t pinned_bytes = 0;
     // autotuned H*v tile shape per (kind, Nup, Ndn), and the timings (ms) of
@@ -337,6 +341,13 @@ int dev_alloc(mo_ed_ctx *ctx, DevBuf &b, size_t bytes);
 int ensure(mo_ed_ctx *ctx, DevBuf &b, size_t bytes);
 // n buffers of `bytes` each in one allocation, which goes with the last of them
 int dev_alloc_slab(mo_ed_ctx *ctx, DevBuf *b, int n, size_t bytes);
+// From a memory pool of the context, for what lives as long as one call.  The
+// pool keeps up to 24 GB (4 GB in a worker context) between calls, where
+// allocating the 20 GB of an eigensolve of 15 million FP32 elements takes 10 ms
+// and freeing it 17.  What idles in it is the driver's to give away: a cudaMalloc
+// of anything else in the process that finds no room takes it (measured: 272 of
+// 276 GB allocated next to a pool that held 20).
+int pool_alloc(mo_ed_ctx *ctx, DevBuf &b, size_t bytes);
 int ensure_pinned(mo_ed_ctx *ctx, size_t bytes);
 // host vector in the reference layout (D contiguous) <-> device vector in the
 // padded layout (ndown rows of stride ld, zero pads); es = element size.

@@ -225,15 +225,15 @@ int lz_setup(mo_ed_ctx *ctx, LzBatch &b, const std::vector<Sector> &secs, int pr
         b.hv_total += b.hv_nitems[r];
         vbytes += 4 * up256(es * (size_t)secs[r].Dpad());
     }
-    // one workspace: kept in the context up to kLzPoolBytes (an allocation
-    // costs more than several steps of a small sector)
+    // one workspace: the context's up to kLzHoldBytes, then from its pool (a
+    // cudaMalloc costs more than several steps of a small sector)
     const size_t ncoef = (size_t)4 * (nstep + 1) * nrun;
     const size_t ocoef = vbytes, oflags = ocoef + up256(sizeof(double) * ncoef), oupd = oflags + up256(sizeof(int) * 2 * nrun);
     const size_t ohv = oupd + up256(sizeof(double) * std::max(1, b.upd_total));
     const size_t total = ohv + up256(sizeof(double) * std::max(1, b.hv_total));
-    DevBuf &ws = total <= kLzPoolBytes ? ctx->lz_pool : b.own;
-    if (int rc = ensure(ctx, ws, total)) return rc;
-    char *base = (char *)ws.p;
+    const bool hold = total <= kLzHoldBytes;
+    if (int rc = hold ? ensure(ctx, ctx->lz_hold, total) : pool_alloc(ctx, b.own, total)) return rc;
+    char *base = (char *)(hold ? ctx->lz_hold.p : b.own.p);
     b.vecs.clear();
     size_t o = 0;
     for (int r = 0; r < nrun; ++r)

@@ -176,9 +176,13 @@ __global__ void k_lz_finalize(const __grid_constant__ LzBatchDev b, int j, int n
         R.a[j] = dot / nrm;
         // for the next update: square roots and divisions are tens of FP64
         // instructions, so not in its threads
-        const double inv = rsqrt_pos(nrm);
-        R.inv[j] = inv;
-        R.cpl[j] = j > 0 ? nrm * inv * R.inv[j - 1] : 0.0;
+        R.inv[j] = rsqrt_by(nrm, rsqrt_pos(nrm));
+        if (j > 0) {
+            const double last = R.nrm[j - 1], q = div_by(nrm, last, rcp_pos(last));
+            R.cpl[j] = sqrt_by(q, rsqrt_pos(q));
+        } else {
+            R.cpl[j] = 0.0;
+        }
         const double tiny = (double)1.e-12f;
         if (j >= 1 && nrm < tiny) {
             *R.nstep_calc = j;

@@ -62,10 +62,11 @@ __device__ __forceinline__ void rcp_pos_n(const double (&d)[N], double (&y)[N])
     }
 }
 
-// s / d, correctly rounded, with r = RN(1 / d): the last step of a division by
-// Markstein's theorem (IBM J. Res. Dev. 34, 1990), three dependent
-// instructions.  Outside the range where nothing under- or overflows it is
-// the division.
+// s / d for d whose reciprocal r is known to an ulp: q = s r and one correction,
+// three dependent instructions.  Half an ulp and little more; correctly rounded
+// (Markstein, IBM J. Res. Dev. 34, 1990) where r = RN(1 / d) and q is within an
+// ulp, as for d of up to 24 significant bits.  Outside the range of s where
+// nothing under- or overflows it is the division.
 __device__ __forceinline__ double div_by(double s, double d, double r)
 {
     if ((unsigned)(((__double2hiint(s) >> 20) & 0x7ff) - 523) > 1000u) return s / d;   // |s| in [2^-500, 2^500]
@@ -79,7 +80,8 @@ __device__ __forceinline__ double widen(float f);
 // the binomial series
 //   (1 - e)^(-1/2) = 1 + e (1/2 + 3/8 e) + O(e^3),  e = 1 - d y0^2, |e| < 2^-20,
 // five dependent FP64 instructions where a square root and a division take
-// tens.  Outside [2^-100, 2^100] (and for d <= 0, non-finite d) it is those.
+// tens, within an ulp (d y0 goes into e with its rounding error).  Outside
+// [2^-100, 2^100] (and for d <= 0, non-finite d) it is those.
 __device__ __forceinline__ double rsqrt_pos(double d)
 {
     if ((unsigned)((int)(__double_as_longlong(d) >> 52) - 923) > 200u) return 1.0 / sqrt(d);
@@ -87,6 +89,20 @@ __device__ __forceinline__ double rsqrt_pos(double d)
     asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(yf) : "f"((float)d));
     const double y0 = widen(yf), e = fma(-(d * y0), y0, 1.0);
     return fma(y0 * e, fma(e, 0.375, 0.5), y0);
+}
+
+// sqrt(d) and 1/sqrt(d) to half an ulp and little more from y = rsqrt_pos(d):
+// one correction each with an exact residual, for d where nothing under- or
+// overflows ([2^-500, 2^500])
+__device__ __forceinline__ double sqrt_by(double d, double y)
+{
+    const double h = d * y;
+    return fma(fma(-h, h, d), 0.5 * y, h);
+}
+__device__ __forceinline__ double rsqrt_by(double d, double y)
+{
+    const double p = d * y, e = fma(-fma(d, y, -p), y, fma(-p, y, 1.0));
+    return fma(0.5 * y, e, y);
 }
 
 // (double)f by integer operations: a conversion instruction takes a slot of

@@ -1,6 +1,6 @@
-// symeig.h -- eigenvalues and eigenvectors of a small dense symmetric matrix
-// on the host: the projected (Rayleigh-Ritz) problem of the thick-restart
-// Lanczos, m <= kMaxNcv.  The reference's eigensolver (PARPACK) also solves
+// symeig.h -- eigenvalues and eigenvectors of small matrices on the host: the
+// projected (Rayleigh-Ritz) problems of the eigensolvers, dense for the thick
+// restarts, tridiagonal or Hessenberg for the long runs (below).  The reference's eigensolver (PARPACK) also solves
 // its projected problem on the host (LAPACK); on GB300 a one-CTA FP64
 // Jacobi of an m = 40 matrix takes ~1.4 ms per call, the host a few tens of
 // microseconds.
@@ -182,7 +182,7 @@ inline void tri_eigvec(int n, const double *d, const double *e, double theta, do
 {
     double scale = std::fabs(theta);
     for (int i = 0; i < n; ++i) scale = std::max(scale, std::fabs(d[i]) + (i + 1 < n ? std::fabs(e[i]) : 0.0));
-    const double tiny = 2.220446049250313e-16 * (scale + 1e-300);
+    const double tiny = 2.220446049250313e-16 * scale + 1e-290;
     std::vector<double> u0(n), u1(n, 0.0), u2(n, 0.0), l(n, 0.0);
     std::vector<char> swp(n, 0);
     double a = d[0] - theta, b = n > 1 ? e[0] : 0.0;     // the row being eliminated: a at k, b at k + 1
@@ -242,7 +242,7 @@ inline void tri_eigvec(int n, const double *d, const double *e, double theta, do
 inline void hess_eigvec(int n, const double *h, int ld, double theta, double scale, double *y,
                         const double *const *prev = nullptr, int nprev = 0)
 {
-    const double tiny = 2.220446049250313e-16 * scale;
+    const double tiny = 2.220446049250313e-16 * scale + 1e-290;
     std::vector<double> u((size_t)n * n, 0.0), l(n, 0.0);   // u row-major
     std::vector<char> swp(n, 0);
     auto U = [&](int i, int j) -> double & { return u[(size_t)i * n + j]; };

@@ -164,6 +164,15 @@ __global__ void k_lz_finalize(const __grid_constant__ LzBatchDev b, int j, int n
     const LzRunDev &R = b.run[blockIdx.x];
     if (*R.active == 0) return;
     two_sums(R.upd_part, R.upd_nitems, R.hv_part, R.hv_nitems, sums);
+    __syncthreads();
+    if (threadIdx.x == 32) {               // next to warp 0, on another sub-partition's FP64 pipe
+        double c = 0.0;
+        if (j > 0) {
+            const double last = R.nrm[j - 1], q = div_by(sums[0], last, rcp_pos(last));
+            c = sqrt_by(q, rsqrt_pos(q));
+        }
+        R.cpl[j] = c;
+    }
     if (threadIdx.x == 0) {
         const double nrm = sums[0], dot = sums[1];
         R.nrm[j] = nrm;
@@ -177,12 +186,6 @@ __global__ void k_lz_finalize(const __grid_constant__ LzBatchDev b, int j, int n
         // for the next update: square roots and divisions are tens of FP64
         // instructions, so not in its threads
         R.inv[j] = rsqrt_by(nrm, rsqrt_pos(nrm));
-        if (j > 0) {
-            const double last = R.nrm[j - 1], q = div_by(nrm, last, rcp_pos(last));
-            R.cpl[j] = sqrt_by(q, rsqrt_pos(q));
-        } else {
-            R.cpl[j] = 0.0;
-        }
         const double tiny = (double)1.e-12f;
         if (j >= 1 && nrm < tiny) {
             *R.nstep_calc = j;

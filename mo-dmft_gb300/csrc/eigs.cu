@@ -11,14 +11,14 @@
 // Comp. 42, 1984: a recurrence whose vectors stay orthogonal to the square
 // root of the rounding unit finds the eigenvalues of the projected operator
 // to the rounding unit).  Rounding errors grow by the ratio at which Ritz
-// values converge; the period is set from the components measured at each
-// reorthogonalisation so that they stay below 2e-5 (FP32) / 1e-11 (FP64).
+// values converge; the period follows the components measured at each
+// reorthogonalisation, towards 2e-5 (FP32) / 1e-11 (FP64) (kryhost.h).
 //
 // The components h that a reorthogonalisation takes out belong to the
 // projected matrix (KryRun::vectors): H Q = Q (T + h) + beta q e^T holds to
 // rounding whatever their size.  Convergence is judged on the symmetric
 // tridiagonal T; the returned vectors are the right eigenvectors of T + h
-// where h matters.
+// where h matters, and their true residual decides whether they are returned.
 //
 // The run is not restarted while its vectors fit (kKryMax, and half the free
 // memory), so it also takes fewer H*v.  A run that fills the room continues
@@ -78,7 +78,7 @@ __device__ __forceinline__ void kry_store(const KryScal &sc, int j, double n2, d
     const double inv = n2 > 0.0 ? rsqrt_pos(n2) : 0.0;
     sc.inv[j] = inv;
     sc.beta[j] = n2 * inv;
-    sc.alpha[j] = n2 > 0.0 ? d * rcp_pos(n2) : 0.0;
+    sc.alpha[j] = n2 > 0.0 ? div_by(d, n2, rcp_pos(n2)) : 0.0;
 }
 
 // the same from the partials of step j

@@ -154,12 +154,13 @@ int mo_ed_multiply_h_mixed_dev(mo_ed_ctx *ctx, int ne_up, int ne_down, const flo
  * times every variant on that sector and keeps the fastest; this call runs
  * the tuning if needed and reports *nvariant variants: shape[4*i..4*i+3] =
  * (rows per item, threads per CTA, CTAs per SM, kernel: 0 k_hv, or k_hv_row
- * with one row per item; 1 the staged kernels k_hv_async and k_hv_wide; 2 / 3
+ * and, in FP64, k_hv_sorted with one row per item; 1 the staged kernels k_hv_async and k_hv_wide; 2 / 3
  * split: k_hv_down over down-spin blocks on 128- / 64-byte row slices, then
  * k_hv_async for the other terms; 4 split: k_hv_down_rows, then k_hv_async or
  * k_hv_wide),
  * ms[i] (negative: does not fit this sector or model), and the *chosen
- * index.  Arrays hold capacity variants.  Pinning a split variant on a model
+ * index.  The list is this build's: a
+ * number stands for another kernel in another one.  Arrays hold capacity variants.  Pinning a split variant on a model
  * whose down-spin blocks do not fit one CTA fails with MO_ED_ERR_ARG. */
 int mo_ed_hv_tuning(mo_ed_ctx *ctx, int ne_up, int ne_down, int dtype, int capacity, int *nvariant,
                     int *shape, float *ms, int *chosen);

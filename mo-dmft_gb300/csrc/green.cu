@@ -602,7 +602,7 @@ namespace moed {
 
 // The eigensolves of ed_solve's sector list (ed_solver.F90:44-60): eig_all
 // [nsector][nev] and the eigenvectors of each sector.  Sectors are
-// independent, and a small sector's thick-restart Lanczos is a chain of
+// independent, and a small sector's Lanczos run is a chain of
 // short dependent launches, so lists of many small sectors are spread over
 // host threads, each driving worker contexts of its own (same device, model
 // and options; own stream and workspace) so that the chains overlap on the
@@ -792,12 +792,13 @@ int mo_ed_delta_new(mo_ed_ctx *ctx, int nwloc, double rmu, const double *Gr, dou
     BandPts bp;
     bp.e = (const double *)ctx->d_hkw.p;
     for (int c = 0; c < 4; ++c) bp.end[c] = ctx->hkw_end[c];
-    // threads per output: enough warps for the chip's 608 sub-partitions
-    // first (few outputs: a CTA or a warp each), then few lanes, because each
+    // threads per output: enough warps for the chip's sub-partitions (four per
+    // SM) first (few outputs: a CTA or a warp each), then few lanes, because each
     // output's divisions and lane sums (~100 FP64 instructions) are issued
     // once per warp
-    auto kern = n <= 304 ? k_delta_new<128> : n <= 2432 ? k_delta_new<32> : k_delta_new<16>;
-    const long long per = n <= 304 ? 128 : n <= 2432 ? 32 : 16;
+    const int few = 2 * ctx->num_sms, some = 16 * ctx->num_sms;
+    auto kern = n <= few ? k_delta_new<128> : n <= some ? k_delta_new<32> : k_delta_new<16>;
+    const long long per = n <= few ? 128 : n <= some ? 32 : 16;
     kern<<<(unsigned)((n * per + 127) / 128), 128, 0, ctx->stream>>>(
         (const double *)ctx->d_hk.p, ctx->nq, bp, rmu, (const double *)dg.p, (double *)dd.p, (double *)dk.p, n);
     MOED_CHECK_LAUNCH(ctx);

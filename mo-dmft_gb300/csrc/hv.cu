@@ -1725,13 +1725,17 @@ static size_t dyn_smem_bytes_async(int ld, const ModelDev &m, const DescGeom &g)
 // ---------------------------------------------------------------------------
 // tile-shape variants and the autotuner
 // ---------------------------------------------------------------------------
-// A variant fixes the kernel (k_hv or k_hv_async), the rows per item R, the CTA
-// size NT and the CTAs per SM the register budget is cut for (MINB).  The
-// k_hv variants compute every element with the same sequence of operations
-// (bit-identical outputs); k_hv_async adds the up-spin terms in the order of
-// the gather schedule, so FP32 outputs of the two kernels agree to rounding.
-// The first H*v of a (kind, Nup, Ndn) shape times each variant on that sector
-// (scratch vectors, CUDA events on the context stream) and keeps the fastest.
+// A variant fixes the kernel, the rows per item R, the CTA size NT and the CTAs
+// per SM the register budget is cut for (MINB).  The kernels add the terms of an
+// element in different orders (k_hv and k_hv_row by column and move, k_hv_async
+// and k_hv_wide as their gather schedules have them, k_hv_sorted the down-spin
+// moves last), so their outputs agree to rounding.  The first H*v of a (kind,
+// Nup, Ndn) shape of kTuneMinElems elements or more times each variant on that
+// sector (scratch vectors, CUDA events on the context stream) and keeps the
+// fastest.  A variant number belongs to these tables, not to the interface:
+// programs that pin one take it from the list of hv_tuning.
+// k_hv_wide<8> has 26 warps: they take the 101 units of 64 columns of a row of
+// 6,435 in four turns, and their 72 registers a thread are 91 % of an SM's.
 struct HvVariant {
     int R, NT, MINB;
     // 0: k_hv, or k_hv_row when R = 1; 1: k_hv_async (double-buffered asynchronous stage);
@@ -1757,7 +1761,7 @@ static const int kNVarF64 = sizeof(kVarF64) / sizeof(kVarF64[0]);
 static const HvVariant &variant(int kind, int v) { return kind == HV_F32 ? kVarF32[v] : kVarF64[v]; }
 static int nvariants(int kind) { return kind == HV_F32 ? kNVarF32 : kNVarF64; }
 
-constexpr long long kTuneMinElems = 1ll << 18;   // smaller sectors take variant 0 untimed
+constexpr long long kTuneMinElems = 1ll << 18;   // smaller sectors take a shape by rule (hv_prepare)
 
 static long long shape_key(int kind, const Sector &s) { return ((long long)kind << 32) | (s.ne_up << 16) | s.ne_down; }
 

@@ -5,9 +5,9 @@
 // arrays of its self-consistency loop: Green's functions, hybridisations,
 // bath parameters), or whose outer loop cannot stand the device-wide
 // synchronisation that cudaFree implies, still needs the Lanczos
-// coefficients of each excitation.  mo_ed_lanczos_iteration allocates its
-// Krylov vectors, coefficients and partial sums on every call;
-// mo_ed_lanczos_iteration_noalloc runs the same kernels on a fixed region
+// coefficients of each excitation.  mo_ed_lanczos_iteration takes its Krylov
+// vectors, coefficients and partial sums from memory that it allocates as they
+// grow; mo_ed_lanczos_iteration_noalloc runs the same kernels on a fixed region
 // that the library reserves statically on every GPU that loads it.
 //
 // The region is kNoAllocBytes (32 MiB) and is held until the process exits.

@@ -62,7 +62,7 @@ int pool_alloc(mo_ed_ctx *ctx, DevBuf &b, size_t bytes)
         props.location.type = cudaMemLocationTypeDevice;
         props.location.id = ctx->device;
         MOED_CUDA(ctx, cudaMemPoolCreate(&ctx->mem_pool, &props));
-        unsigned long long keep = (ctx->worker ? 4ull : 24ull) << 30;
+        unsigned long long keep = pool_keep(ctx);
         MOED_CUDA(ctx, cudaMemPoolSetAttribute(ctx->mem_pool, cudaMemPoolAttrReleaseThreshold, &keep));
     }
     if (bytes == 0) bytes = 16;

@@ -348,6 +348,7 @@ int dev_alloc_slab(mo_ed_ctx *ctx, DevBuf *b, int n, size_t bytes);
 // of anything else in the process that finds no room takes it (measured: 272 of
 // 276 GB allocated next to a pool that held 20).
 int pool_alloc(mo_ed_ctx *ctx, DevBuf &b, size_t bytes);
+inline size_t pool_keep(const mo_ed_ctx *ctx) { return (size_t)(ctx->worker ? 4 : 24) << 30; }
 int ensure_pinned(mo_ed_ctx *ctx, size_t bytes);
 // host vector in the reference layout (D contiguous) <-> device vector in the
 // padded layout (ndown rows of stride ld, zero pads); es = element size.

@@ -239,7 +239,9 @@ int lz_setup(mo_ed_ctx *ctx, LzBatch &b, const std::vector<Sector> &secs, int pr
     const size_t ohv = oupd + up256(sizeof(double) * std::max(1, b.upd_total));
     const size_t total = ohv + up256(sizeof(double) * std::max(1, b.hv_total));
     const bool hold = total <= kLzHoldBytes;
-    if (int rc = hold ? ensure(ctx, ctx->lz_hold, total) : pool_alloc(ctx, b.own, total)) return rc;
+    if (int rc = hold ? ensure(ctx, ctx->lz_hold, total)
+                      : total <= pool_keep(ctx) ? pool_alloc(ctx, b.own, total) : dev_alloc(ctx, b.own, total))
+        return rc;
     char *base = (char *)(hold ? ctx->lz_hold.p : b.own.p);
     b.vecs.clear();
     size_t o = 0;

@@ -1302,8 +1302,8 @@ k_hv_row(const __grid_constant__ HvBatch<TA> batch, const ModelDev *__restrict__
 // Bound by shared-memory wavefronts and their latency (ncu, 15 million
 // elements: 55 % of the LSU pipe, DRAM at 19 %): a slot serves the lanes that
 // have a move in it, 58 % of them.  Ground sector of 3 orbitals x 4 levels, 41
-// million elements: R = 8 after k_hv_down_rows 322 us (of it k_hv_wide 218; 320
-// with x . y in FP32 over the row, whose register ptxas then did not spill),
+// million elements: R = 8 after k_hv_down_rows 322 us (320, of it k_hv_wide 216,
+// with x . y in FP32 over the row: 12 bytes of spills now, 4 then),
 // two CTAs of R = 4 fused 345 us, R = 4 split 335 us; k_hv_async<SPLIT, 4> 463.
 // Tried and not kept: more slots or moves in flight at fewer warps (350-550
 // us, registers), skipping the lanes without a move by predicate (the same).
